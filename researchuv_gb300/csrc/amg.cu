@@ -28,6 +28,7 @@
 #include <memory>
 
 #include "system.cuh"
+#include "team.cuh"
 
 namespace ruv {
 namespace {
@@ -2569,6 +2570,28 @@ class AmgPrecond final : public SepPrecond {
   void bind(Ctx& ctx, void* r, void* z, bool) override { amg_bind(ctx, H_, static_cast<float*>(r), static_cast<float*>(z)); }
   int apply(Ctx& ctx, const int32_t* done) override { return amg_apply(ctx, H_, done); }
   const int* error_flag() const override { return H_->err; }
+  void team(TeamPrecond& out) const override {
+    const int K = (int)H_->lv.size();
+    if (H_->k_levels > 0 || K > kTeamMaxLevels) return;
+    out.kind = 1;
+    TeamAmg& M = out.amg;
+    M.final_lvl = H_->final_lvl;
+    M.fac_off = H_->fac_off;
+    M.fac = H_->fac;
+    M.alpha_c = H_->alpha_c;
+    // lanes a row needs so that each has at most about 16 entries
+    auto lanes = [](int64_t nnz, int64_t n) {
+      const double avg = n > 0 ? (double)nnz / (double)n : 1.0;
+      return avg <= 16 ? 0 : avg <= 32 ? 1 : avg <= 64 ? 2 : 3;
+    };
+    for (int k = 0; k < K; ++k) {
+      const AmgLevelDev& L = H_->lv[k];
+      const int64_t nc = k + 1 < K ? H_->lv[k + 1].n : 0;
+      M.lv[k] = TeamLevel{L.chart_row, L.rp, L.cols, L.c16, L.cbase, !L.c16 ? 0 : L.rowrel ? 2 : 1, L.vals, L.dinv,
+                          L.poff, L.roff, L.pc, L.rc, L.agg, L.pv, L.rv, L.b, L.x, L.y, L.t, L.smoothed ? 1 : 0,
+                          lanes(L.nnz, L.n), lanes(L.n_pnnz, nc), lanes(L.n_pnnz, L.n)};
+    }
+  }
 
  private:
   AmgHierarchy* H_ = nullptr;

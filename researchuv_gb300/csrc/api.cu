@@ -238,7 +238,10 @@ ruv_status ruv_ctx_create(ruv_ctx** out, int32_t device) {
   ctx->c.device = device;
   ctx->c.sm_count = prop.multiProcessorCount;
   // launch-shape overrides for the tuner (RUV_LPR, RUV_UNROLL, RUV_TILE_ROWS)
-  if (const char* e = std::getenv("RUV_LPR")) ctx->c.lanes_per_row = std::atoi(e);
+  if (const char* e = std::getenv("RUV_LPR")) {
+    ctx->c.lanes_per_row = std::atoi(e);
+    ctx->c.shape_forced = ctx->c.lanes_per_row > 0;
+  }
   if (const char* e = std::getenv("RUV_UNROLL")) ctx->c.unroll = std::atoi(e);
   if (const char* e = std::getenv("RUV_TILE_ROWS")) ctx->c.tile_rows = std::max(32, std::atoi(e));
   if (cudaSetDevice(device) != cudaSuccess) return RUV_ERR_NO_DEVICE;
@@ -263,6 +266,14 @@ void ruv_ctx_destroy(ruv_ctx* ctx) {
   cudaStreamSynchronize(ctx->c.stream);
   cudaStreamSynchronize(ctx->c.side);
   ctx->c.ws.release();
+  for (cudaStream_t st : ctx->c.team_stream)
+    if (st) {
+      cudaStreamSynchronize(st);
+      cudaStreamDestroy(st);
+    }
+  for (cudaEvent_t e : ctx->c.team_done)
+    if (e) cudaEventDestroy(e);
+  if (ctx->c.team_go) cudaEventDestroy(ctx->c.team_go);
   cudaStreamDestroy(ctx->c.stream);
   cudaStreamDestroy(ctx->c.side);
   for (cudaEvent_t* e : copy_events(ctx->c)) cudaEventDestroy(*e);
@@ -683,6 +694,9 @@ ruv_status ruv_lscm_solve_batch_keep_metric(ruv_ctx* ctx, const ruv_lscm_batch* 
     so.precision = o.precision;
     so.tol = o.tol;
     so.max_iter = o.max_cg_iter > 0 ? o.max_cg_iter : 16384;
+    // (charts whose area iteration does not settle carry the last bits of these solves into their
+    // results: the order of their sums stays the launch-per-step loop's)
+    so.teams = false;
     auto r1 = pcg_solve(c, sys, yb, so);
     double* b_saved = sys.b;
     sys.b = u;

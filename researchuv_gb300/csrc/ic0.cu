@@ -39,6 +39,7 @@
 #include <memory>
 
 #include "system.cuh"
+#include "team.cuh"
 
 namespace ruv {
 namespace {
@@ -237,9 +238,11 @@ __global__ void __launch_bounds__(kIcThreads) k_factor(const int64_t* __restrict
 }
 
 __global__ void k_t_values(int64_t nnz, const int64_t* __restrict__ tsrc, const double* __restrict__ lv,
-                           double* __restrict__ tv, float* __restrict__ tv32, float* __restrict__ lv32) {
+                           double* __restrict__ tv, float* __restrict__ tv32, float* __restrict__ lv32,
+                           int64_t n, const int64_t* __restrict__ lptr, double* __restrict__ inv) {
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nnz) return;
+  if (e >= nnz) return;  // (n <= nnz: every row has its pivot)
+  if (e < n) inv[e] = 1.0 / lv[lptr[e + 1] - 1];
   const double v = lv[tsrc[e]];
   tv[e] = v;
   tv32[e] = (float)v;
@@ -619,7 +622,7 @@ struct Factor {
   int64_t n = 0, nnz = 0;
   int64_t *lptr = nullptr, *tptr = nullptr, *tsrc = nullptr;
   int32_t *lc = nullptr, *tc = nullptr;
-  double *lv = nullptr, *tv = nullptr;
+  double *lv = nullptr, *tv = nullptr, *inv = nullptr;  // inv: 1 / pivot of each row
   float *lv32 = nullptr, *tv32 = nullptr;
   int32_t *frows = nullptr, *flev = nullptr, *fnl = nullptr;
   int32_t *brows = nullptr, *blev = nullptr, *bnl = nullptr;
@@ -677,6 +680,7 @@ Factor factor_pattern(Ctx& ctx, const DevSystem& sys, const std::string& tag, in
   F.lv32 = ws.get<float>(tag + ".lv32", std::max<int64_t>(nnz, 1));
   F.tv32 = ws.get<float>(tag + ".tv32", std::max<int64_t>(nnz, 1));
   F.tptr = ws.get<int64_t>(tag + ".tptr", N + 1);
+  F.inv = ws.get<double>(tag + ".inv", std::max<int64_t>(N, 1));
   if (N > 0) {
     k_l_fill<<<g, kIcThreads, 0, s>>>(N, sys.row_ptr, sys.cols, sys.vals, F.lptr, F.lc, F.lv, flags);
     RUV_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * N, s));
@@ -786,7 +790,8 @@ void factor_values(Ctx& ctx, const DevSystem& sys, Factor& F, int* flags) {
     count_launches(1);
   }
   if (F.nnz > 0) {
-    k_t_values<<<div_up(F.nnz, 256), 256, 0, s>>>(F.nnz, F.tsrc, F.lv, F.tv, F.tv32, F.lv32);
+    k_t_values<<<div_up(F.nnz, 256), 256, 0, s>>>(F.nnz, F.tsrc, F.lv, F.tv, F.tv32, F.lv32, F.n,
+                                                             F.lptr, F.inv);
     count_launches(1);
   }
   RUV_LAUNCH_CHECK();
@@ -889,6 +894,28 @@ class Ic0Precond final : public SepPrecond {
     return nrhs_ == 2 ? run<float, 2>(ctx, done) : run<float, 1>(ctx, done);
   }
   const int* error_flag() const override { return F_.tickets ? F_.tick + 2 : nullptr; }
+  void team(TeamPrecond& out) const override {
+    if (F_.tickets) return;
+    out.kind = 2;
+    TeamIc0& I = out.ic0;
+    I.frows = F_.frows;
+    I.flev = F_.flev;
+    I.fnl = F_.fnl;
+    I.brows = F_.brows;
+    I.blev = F_.blev;
+    I.bnl = F_.bnl;
+    I.lptr = F_.lptr;
+    I.tptr = F_.tptr;
+    I.lc = F_.lc;
+    I.tc = F_.tc;
+    I.lv = fp64_ ? static_cast<const void*>(F_.lv) : F_.lv32;
+    I.tv = fp64_ ? static_cast<const void*>(F_.tv) : F_.tv32;
+    I.inv = F_.inv;
+    I.y = y_;
+    I.zp = zp_;
+    I.to_orig = to_orig_;
+    I.width = F_.max_chart_rows / std::max(F_.max_levels, 1);
+  }
   int levels() const { return F_.max_levels; }
   int colours() const { return n_colours_; }
   const Factor& factor() const { return F_; }

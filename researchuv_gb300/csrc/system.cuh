@@ -41,6 +41,7 @@ struct SolveOpts {
   ruv_precision precision = RUV_PREC_FP64;
   double tol = 1e-12;
   int64_t max_iter = 16384;
+  bool teams = true;  // charts may be solved by the team kernels (team.cu)
 };
 
 struct ChartResult {
@@ -56,8 +57,11 @@ struct Ctx;
 // steps: z = M^-1 r for every chart whose CG is still running.  Set up from an assembled
 // system on construction; bound once to the CG's r and z; apply() only enqueues launches
 // (capturable in a CUDA graph) and returns how many.
+struct TeamPrecond;
 struct SepPrecond {
   virtual ~SepPrecond() = default;
+  // what a team kernel needs to apply it itself (after bind; team.cuh); left alone: it cannot
+  virtual void team(TeamPrecond&) const {}
   virtual bool native_fp64() const = 0;  // applies in FP64 under the FP64 loop (else FP32 copies)
   virtual bool flexible() const = 0;     // varies between applications: flexible-CG beta
   virtual void bind(Ctx& ctx, void* r, void* z, bool fp64) = 0;
@@ -184,6 +188,12 @@ struct Ctx {
   cudaEvent_t ev_part[DevBatch::kMaxParts] = {};
   Workspace ws;
   PinnedHost pinned;
+  // the team solver (team.cu): its chart order, and streams for its launches to run side by side
+  PinnedHost team_pinned;
+  cudaStream_t team_stream[4] = {};
+  cudaEvent_t team_go = nullptr, team_done[4] = {};
+  void team_streams(int n);  // makes sure that the first n exist
+  bool shape_forced = false;  // RUV_LPR: the SpMV shape of the launch-per-step loop is chosen
   std::string last_error;
   // the last batch's assembled system (for ruv_export_chart_system)
   DevSystem last_sys;
