@@ -20,7 +20,7 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 CU_SOURCES = ["adjoint.cu", "amg.cu", "api.cu", "assemble.cu", "ic0.cu", "pcg.cu", "prep_gpu.cu", "scan.cu",
               "team.cu"]
 CXX_SOURCES = ["prep.cpp"]
-HEADERS = ["common.cuh", "fp64rn.cuh", "pcg.cuh", "system.cuh", "team.cuh", "ruv_internal.h"]
+HEADERS = ["common.cuh", "fp64rn.cuh", "pcg.cuh", "system.cuh", "team.cuh", "team_dev.cuh", "ruv_internal.h"]
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 

@@ -74,12 +74,17 @@ long long env_level_entry(const char* knob, int k) {
   return 0;
 }
 
-// Rows per V-cycle tile of level k: the k-th entry of RUV_AMG_TILE (0 or missing: the default
-// above; 64 to 65536 taken).
-int64_t level_tile_rows(int k) {
+// Rows per V-cycle tile of level k with n rows: the k-th entry of RUV_AMG_TILE (0 or missing: the
+// default above; 64 to 65536 taken).  A level too small to give every SM four tiles of that size gets
+// smaller ones, down to 64 rows: a CTA walks its tile's rows in passes of 64 to 256, each a chain of
+// three dependent loads, so a 1024^2 field's coarse levels (44,000 rows and fewer in 512-row tiles)
+// took 13-21 us a kernel with most SMs idle.
+int64_t level_tile_rows(int k, int64_t n, int sm_count) {
   const long long v = env_level_entry("RUV_AMG_TILE", k);
   if (v >= 64 && v <= 65536) return v;
-  return k == 0 ? kLevelTile0 : kLevelTile;
+  int64_t tile = k == 0 ? kLevelTile0 : kLevelTile;
+  while (tile > 64 && n < 4 * tile * sm_count) tile /= 2;
+  return tile;
 }
 
 __device__ __forceinline__ int64_t find_chart64(const int64_t* off, int64_t n_charts, int64_t i) {
@@ -1605,10 +1610,16 @@ __global__ void __launch_bounds__(kDirect) k_direct_solve(const int32_t* __restr
   float s[NR];
 #pragma unroll
   for (int k = 0; k < NR; ++k) s[k] = 0.0f;
-  for (int j = 0; j < m; ++j) {
-    const float a = Ainv[j * m + i];
+  // (sixteen columns loaded at a time, added in order: one load in flight took 14 us for one chart)
+  for (int j0 = 0; j0 < m; j0 += 16) {
+    float a[16];
 #pragma unroll
-    for (int k = 0; k < NR; ++k) s[k] += a * bs[k][j];
+    for (int q = 0; q < 16; ++q) a[q] = j0 + q < m ? __ldg(Ainv + (j0 + q) * m + i) : 0.0f;
+#pragma unroll
+    for (int q = 0; q < 16; ++q)
+      if (j0 + q < m)
+#pragma unroll
+        for (int k = 0; k < NR; ++k) s[k] += a[q] * bs[k][j0 + q];
   }
 #pragma unroll
   for (int k = 0; k < NR; ++k) x[NR * (r0 + i) + k] = s[k];
@@ -2144,7 +2155,7 @@ AmgHierarchy* amg_setup(Ctx& ctx, const DevSystem& sys, bool smooth, std::string
   for (int k = 0; k < K; ++k) {
     AmgLevelDev& L = H->lv[k];
     const std::string tag = "amg.v" + std::to_string(k);
-    const int64_t tile = level_tile_rows(k);
+    const int64_t tile = level_tile_rows(k, L.n, ctx.sm_count);
     for (int which = 0; which < 2; ++which) {
       std::vector<int64_t> tab, ctile(NC + 1, 0);
       std::vector<int32_t> tch;
@@ -2579,10 +2590,10 @@ class AmgPrecond final : public SepPrecond {
     M.fac_off = H_->fac_off;
     M.fac = H_->fac;
     M.alpha_c = H_->alpha_c;
-    // lanes a row needs so that each has at most about 16 entries
+    // lanes a row needs so that each has at most a sweep of eight entries and a half
     auto lanes = [](int64_t nnz, int64_t n) {
       const double avg = n > 0 ? (double)nnz / (double)n : 1.0;
-      return avg <= 16 ? 0 : avg <= 32 ? 1 : avg <= 64 ? 2 : 3;
+      return avg <= 12 ? 0 : avg <= 24 ? 1 : avg <= 48 ? 2 : 3;
     };
     for (int k = 0; k < K; ++k) {
       const AmgLevelDev& L = H_->lv[k];

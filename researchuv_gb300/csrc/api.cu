@@ -243,7 +243,10 @@ ruv_status ruv_ctx_create(ruv_ctx** out, int32_t device) {
     ctx->c.shape_forced = ctx->c.lanes_per_row > 0;
   }
   if (const char* e = std::getenv("RUV_UNROLL")) ctx->c.unroll = std::atoi(e);
-  if (const char* e = std::getenv("RUV_TILE_ROWS")) ctx->c.tile_rows = std::max(32, std::atoi(e));
+  if (const char* e = std::getenv("RUV_TILE_ROWS")) {
+    ctx->c.tile_rows = std::max(32, std::atoi(e));
+    ctx->c.tile_set = true;
+  }
   if (cudaSetDevice(device) != cudaSuccess) return RUV_ERR_NO_DEVICE;
   if (cudaStreamCreateWithFlags(&ctx->c.stream, cudaStreamNonBlocking) != cudaSuccess) return RUV_ERR_LAUNCH;
   bool ok = cudaStreamCreateWithFlags(&ctx->c.side, cudaStreamNonBlocking) == cudaSuccess;

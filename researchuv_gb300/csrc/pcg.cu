@@ -1279,9 +1279,20 @@ void dispatch_pcg(Shape sh, Ctx& ctx, DevSystem& sys, double* x64, const SolveOp
 
 TileTable make_tiles(const std::vector<int64_t>& chart_row, int64_t tile_rows);
 
-Tiles upload_tiles(Ctx& ctx, const DevSystem& sys, const std::string& tag) {
+// Rows per tile of a solve: the context's, or in the mixed loop, where none was chosen and a system is
+// too small to give every SM four tiles of that size, down to 128.  (The FP64 loop keeps its tiles: its
+// block sums occupy the FP64 pipe, and 128-row tiles took a 89,401-row chart from 27 to 36 us an
+// iteration.)
+int64_t solve_tile_rows(const Ctx& ctx, const DevSystem& sys, bool mixed) {
+  int64_t tile = ctx.tile_rows;
+  if (mixed && !ctx.tile_set)
+    while (tile > 128 && sys.n_rows < 4 * tile * ctx.sm_count) tile /= 2;
+  return tile;
+}
+
+Tiles upload_tiles(Ctx& ctx, const DevSystem& sys, const std::string& tag, int64_t tile_rows) {
   cudaStream_t s = ctx.stream;
-  TileTable TT = make_tiles(sys.h_chart_row, ctx.tile_rows);
+  TileTable TT = make_tiles(sys.h_chart_row, tile_rows);
   const int64_t NTL = (int64_t)TT.chart.size(), NC = sys.n_charts;
   int64_t* d_tab = ctx.ws.get<int64_t>(tag + ".tab", 2 * NTL);
   int32_t* d_chart = ctx.ws.get<int32_t>(tag + ".tchart", NTL);
@@ -1513,7 +1524,7 @@ void narrow_columns(Ctx& ctx, DevSystem& sys) {
 double bench_spmv(Ctx& ctx, DevSystem& sys, bool mixed, int reps, int n_buffers, double* bytes,
                   double* stream_bytes) {
   narrow_columns(ctx, sys);
-  Tiles T = upload_tiles(ctx, sys, "bench");
+  Tiles T = upload_tiles(ctx, sys, "bench", ctx.tile_rows);
   const Shape sh = pick_shape(ctx, sys);
   const double N = (double)sys.n_rows, NNZ = (double)sys.nnz, nr = (double)sys.nrhs;
   const double vb = mixed ? 4.0 : 8.0;
@@ -1550,7 +1561,7 @@ TuneResult autotune_spmv(Ctx& ctx, DevSystem& sys, bool mixed, int reps) {
     ctx.tile_rows = tr;
     for (int tma = 0; tma < n_tma; ++tma) {
       ctx.spmv_tma = tma;
-      Tiles T = upload_tiles(ctx, sys, "tune");
+      Tiles T = upload_tiles(ctx, sys, "tune", ctx.tile_rows);
       if (T.n == 0) break;
       for (const Shape& sh : shapes) {
         double ms = sys.nrhs == 2 ? (mixed ? dispatch_time<float, 2>(sh, ctx, sys, T, reps, 2, true)
@@ -1564,6 +1575,7 @@ TuneResult autotune_spmv(Ctx& ctx, DevSystem& sys, bool mixed, int reps) {
     ctx.lanes_per_row = best.lpr;
     ctx.unroll = best.unroll;
     ctx.tile_rows = best.tile_rows;
+    ctx.tile_set = true;
     ctx.spmv_tma = best.tma;
   } else {
     ctx.tile_rows = saved_tile;
@@ -1579,7 +1591,7 @@ std::vector<ChartResult> pcg_solve(Ctx& ctx, DevSystem& sys, double* x, const So
     throw Error{RUV_ERR_BAD_INPUT, "unknown preconditioner"};
   const int64_t NC = sys.n_charts;
   narrow_columns(ctx, sys);
-  Tiles T = upload_tiles(ctx, sys, "pcg");
+  Tiles T = upload_tiles(ctx, sys, "pcg", o.teams ? solve_tile_rows(ctx, sys, o.precision == RUV_PREC_MIXED) : ctx.tile_rows);
   ChartState* st = ctx.ws.get<ChartState>("pcg.state", NC);
   int* n_active = ctx.ws.get<int>("pcg.nactive", 1);
   const Shape sh = pick_shape(ctx, sys);

@@ -41,7 +41,7 @@ struct SolveOpts {
   ruv_precision precision = RUV_PREC_FP64;
   double tol = 1e-12;
   int64_t max_iter = 16384;
-  bool teams = true;  // charts may be solved by the team kernels (team.cu)
+  bool teams = true;  // charts may be solved by the team kernels (team.cu), tiles follow the system's size
 };
 
 struct ChartResult {
@@ -201,6 +201,7 @@ struct Ctx {
   int lanes_per_row = 0;   // SpMV sub-warp width (0 = from the row-length profile)
   int unroll = 0;          // SpMV rows in flight per sub-warp (0 = from the shape)
   int tile_rows = 1024;    // rows per CTA tile (the autotuner's pick on the disks and the height fields)
+  bool tile_set = false;   // tile_rows was chosen (RUV_TILE_ROWS, the autotuner): taken for every system
   // the bulk-copy SpMV (k_spmv_tma): 0 off (the default: on the 4096-disk step the CSR-vector
   // kernel's iteration ran faster), 1 on; the autotuner chooses it, RUV_SPMV_TMA=0/1 overrides
   int spmv_tma = 0;

@@ -17,7 +17,7 @@
 // one lane per CTA from the same partial sums in the same order, so every CTA of a team decides
 // alike and results do not depend on timing.  (FP64 adds have 64 clocks of latency and 1.6 results
 // per clock and SM here: a reduction's last steps and the scalar divisions stay in one warp.)
-#include "team.cuh"
+#include "team_dev.cuh"
 
 #include <algorithm>
 #include <cstdlib>
@@ -28,9 +28,6 @@ namespace {
 constexpr int kTeamThreads = 512;
 constexpr int kTeamWarps = kTeamThreads / 32;
 constexpr int kTeamMaxCtas = 16;
-constexpr float kTeamOmega = 2.0f / 3.0f;  // the V-cycle's Jacobi weight (amg.cu kOmega)
-constexpr int kTeamDirect = 64;            // rows solved by the dense inverse (amg.cu kDirect)
-
 struct TeamShared {
   ChartState st;                    // lane 0's scalars (the same bits in every CTA of the team)
   double part[2][2][kTeamWarps];    // [buffer][value][warp], as S
@@ -71,116 +68,6 @@ __device__ __forceinline__ void st_async(const unsigned long long* p, const uint
   asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(d),
                "l"(v), "r"(m)
                : "memory");
-}
-
-// 1 / d for a finite d whose reciprocal is normal: an FP32 seed of the significand and two Newton
-// steps, within about an ulp.  d outside that goes to the division.
-__device__ __forceinline__ double rcp64(double d) {
-  const uint64_t u = (uint64_t)__double_as_longlong(d);
-  const int e = (int)(u >> 52) & 0x7ff;
-  if (e < 2 || e > 2044) return 1.0 / d;
-  const double m = __longlong_as_double((long long)((u & 0x000fffffffffffffull) | 0x3ff0000000000000ull));
-  double r = (double)(1.0f / (float)m);
-  r = fma(r, fma(-m, r, 1.0), r);
-  r = fma(r, fma(-m, r, 1.0), r);
-  const uint64_t scale = ((uint64_t)(2046 - e) << 52) | (u & 0x8000000000000000ull);
-  return r * __longlong_as_double((long long)scale);
-}
-// a / b from r = rcp64(b): the product and one correction by its exact remainder (the rounding of
-// the division up to the last bit; a chain of three FP64 operations, where the division takes ten).
-// Quotients that leave the normal range go to the division.
-__device__ __forceinline__ double div_by(double a, double b, double r) {
-  const double q = a * r;
-  if (a == 0.0) return q;
-  const int e = (int)((uint64_t)__double_as_longlong(q) >> 52) & 0x7ff;
-  if (e < 64 || e > 1982) return a / b;
-  return fma(fma(-q, b, a), r, q);
-}
-__device__ __forceinline__ double div64(double a, double b) { return div_by(a, b, rcp64(b)); }
-
-// A sum in double-float: an unevaluated FP32 pair (48 bits).  The mixed loop's scalars are formed in
-// these -- its partial sums are FP32, its vectors take alpha and beta rounded to FP32 -- because a
-// dependent FP64 operation takes 64 clocks here and an FP32 one four (a reduction with its
-// division: 2,000 clocks in FP64 against 700).
-struct Pair {
-  float h, l;
-  __device__ __forceinline__ double f64() const { return (double)h + (double)l; }
-};
-__device__ __forceinline__ Pair pair_of(float a) { return Pair{a, 0.0f}; }
-__device__ __forceinline__ Pair pair_of(double a) {
-  Pair r;
-  split_f64(a, r.h, r.l);
-  return r;
-}
-__device__ __forceinline__ Pair pair_add(Pair a, Pair b) {
-  float s, e;
-  two_sum(a.h, b.h, s, e);
-  e += a.l + b.l;
-  const float h = s + e;
-  return Pair{h, e - (h - s)};
-}
-__device__ __forceinline__ Pair pair_div(Pair a, Pair b) {
-  const float q1 = a.h / b.h;
-  if (!(fabsf(q1) < 3e38f) || q1 == 0.0f) return Pair{q1, 0.0f};
-  // the remainder a - q1 b to twice FP32, and its quotient
-  const float p = q1 * b.h, pe = fmaf(q1, b.h, -p);
-  const float q2 = ((a.h - p) - pe + (a.l - q1 * b.l)) / b.h;
-  const float h = q1 + q2;
-  return Pair{h, q2 - (h - q1)};
-}
-__device__ __forceinline__ Pair pair_mul(Pair a, Pair b) {
-  const float p = a.h * b.h;
-  const float e = fmaf(a.h, b.h, -p) + (a.h * b.l + a.l * b.h);
-  const float h = p + e;
-  return Pair{h, e - (h - p)};
-}
-// What a reduction's totals and the scalars formed from them are held in.
-template <class S>
-struct ScalarOf {
-  using type = double;
-};
-template <>
-struct ScalarOf<float> {
-  using type = Pair;
-};
-__device__ __forceinline__ double sc_add(double a, double b) { return a + b; }
-__device__ __forceinline__ Pair sc_add(Pair a, Pair b) { return pair_add(a, b); }
-__device__ __forceinline__ double sc_div(double a, double b) { return div64(a, b); }
-__device__ __forceinline__ Pair sc_div(Pair a, Pair b) { return pair_div(a, b); }
-__device__ __forceinline__ double sc_neg_mul(double a, double b) { return -a * b; }
-__device__ __forceinline__ Pair sc_neg_mul(Pair a, Pair b) { return pair_mul(Pair{-a.h, -a.l}, b); }
-__device__ __forceinline__ double sc_hi(double a) { return a; }
-__device__ __forceinline__ float sc_hi(Pair a) { return a.h; }
-__device__ __forceinline__ bool vanishes(double a) { return fabs(a) <= 1e-300; }
-__device__ __forceinline__ bool vanishes(Pair a) { return a.h == 0.0f; }
-__device__ __forceinline__ double sc_zero(double) { return 0.0; }
-__device__ __forceinline__ Pair sc_zero(Pair) { return Pair{0.0f, 0.0f}; }
-__device__ __forceinline__ double sc_from(double, double v) { return v; }
-__device__ __forceinline__ Pair sc_from(Pair, double v) { return pair_of(v); }
-__device__ __forceinline__ double sc_f64(double a) { return a; }
-__device__ __forceinline__ double sc_f64(Pair a) { return a.f64(); }
-__device__ __forceinline__ double sc_shfl(double a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
-__device__ __forceinline__ Pair sc_shfl(Pair a, int o) {
-  return Pair{__shfl_xor_sync(0xffffffffu, a.h, o), __shfl_xor_sync(0xffffffffu, a.l, o)};
-}
-__device__ __forceinline__ unsigned long long sc_bits(double a) { return (unsigned long long)__double_as_longlong(a); }
-__device__ __forceinline__ unsigned long long sc_bits(Pair a) {
-  return ((unsigned long long)__float_as_uint(a.h) << 32) | __float_as_uint(a.l);
-}
-__device__ __forceinline__ double sc_of_bits(double, unsigned long long b) { return __longlong_as_double((long long)b); }
-__device__ __forceinline__ Pair sc_of_bits(Pair, unsigned long long b) {
-  return Pair{__uint_as_float((unsigned)(b >> 32)), __uint_as_float((unsigned)b)};
-}
-// sqrt(rr) <= norm (norm2 = square_of(norm)); an FP32 sum of squares against the FP32 square
-__device__ __forceinline__ double square_of(double, double norm) {
-  return norm > 1e-140 && norm < 1e140 ? norm * norm : -1.0;
-}
-__device__ __forceinline__ float square_of(float, double norm) {
-  return norm > 1e-18 && norm < 1e18 ? (float)(norm * norm) : -1.0f;
-}
-template <class R>
-__device__ __forceinline__ bool at_most(R rr, double norm, R norm2) {
-  return norm2 > R(0) ? rr <= norm2 : sqrt((double)rr) <= norm;
 }
 
 struct Team {
@@ -261,148 +148,186 @@ __device__ __forceinline__ int team_reduce(Team& tm, TeamShared& sh, const T (&v
   return sh.flag;
 }
 
-// A CSR operator's column stream (see ColsWide, ColsNarrow, ColsRowRel).
-struct Cols {
-  const int32_t* c32;
-  const uint16_t* c16;
-  int kind;
-  int32_t cb;
-  __device__ __forceinline__ int32_t base(int32_t i) const { return kind == 2 ? i - kRowRelBias : cb; }
-  __device__ __forceinline__ int32_t at(int32_t e, int32_t rb) const {
-    return kind ? rb + (int32_t)__ldg(c16 + e) : __ldg(c32 + e);
-  }
+// A step over rows [r0 + q, r0 + end) of a level, q from place's on: for each, s = sum_e w(e) get(col(e,
+// row)) by 2^ll lanes, then fin(row, early, s) in the row's first lane, where early(row) was loaded
+// beside the gathers.  Offsets and entries do not change, so the first row's are loaded before the
+// barrier in front of the step is waited for.  Trip counts are uniform in a warp.
+struct Place {
+  int32_t q, end, step;
+  int sub, ll;
 };
-
-// sum_e vals[e] get(col(e)) of one row, eight entries in flight (a mesh Laplacian's row in one
-// sweep), entry order.
-template <class S, int NR, class Get>
-__device__ __forceinline__ V<S, NR> row_dot(const int32_t* rp, const Cols& cols, const S* vals, int32_t i, Get get) {
-  const int32_t lo = __ldg(rp + i), hi = __ldg(rp + i + 1), rb = cols.base(i);
-  V<S, NR> s;
-#pragma unroll
-  for (int c = 0; c < NR; ++c) s.c[c] = S(0);
-  for (int32_t e0 = lo; e0 < hi; e0 += 8) {
-    S a[8];
-    int32_t j[8];
+template <int NR, class Ptr, class Col, class W, class G, class Early, class Fin, class Bar>
+__device__ __forceinline__ void level_step(const Place& at, int32_t r0, Ptr ptr, Col col, W w, G get, Early early, Fin fin,
+                                           Bar bar) {
+  using Vf = V<float, NR>;
+  const int lanes = 1 << at.ll, off = at.q & ((32 >> at.ll) - 1);
+  int32_t lo, hi, j[8];
+  float a[8];
+  auto entries = [&](int32_t e0, int32_t i) {
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      const bool in = e0 + k < hi;
-      a[k] = in ? __ldg(vals + e0 + k) : S(0);
-      j[k] = in ? cols.at(e0 + k, rb) : -1;
+      const int32_t e = e0 + k * lanes;
+      const bool in = e < hi;
+      a[k] = in ? w(e) : 0.0f;
+      j[k] = in ? col(e, i) : -1;
     }
+  };
+  auto head = [&](int32_t q) {
+    const bool valid = q < at.end;
+    lo = valid ? (int32_t)__ldg(ptr + r0 + q) : 0;
+    hi = valid ? (int32_t)__ldg(ptr + r0 + q + 1) : 0;
+    entries(lo + at.sub, r0 + q);
+  };
+  head(at.q);
+  bar();
+  for (int32_t g = at.q - off; g < at.end; g += at.step) {
+    const int32_t q = g + off, i = r0 + q;
+    if (q != at.q) head(q);
+    decltype(early(0)) x;
+    Vf v[8], s;
+    if (q < at.end) x = early(i);
 #pragma unroll
     for (int k = 0; k < 8; ++k)
-      if (j[k] >= 0) {
-        const V<S, NR> g = get(j[k]);
-#pragma unroll
-        for (int c = 0; c < NR; ++c) s.c[c] += a[k] * g.c[c];
-      }
-  }
-  return s;
-}
-
-// For each of the n rows from row r0 on: s = sum_e w(e) get(col(e, row)), by 2^ll lanes, then
-// fin(row, s) in the row's first lane.  Trip counts are uniform, so every lane is in the shuffles.
-template <int NR, class Ptr, class Col, class W, class G, class Fin>
-__device__ __forceinline__ void level_rows(const Team& tm, int32_t r0, int32_t n, int ll, Ptr ptr, Col col, W w, G get,
-                                           Fin fin) {
-  const int lanes = 1 << ll, sub = tm.id & (lanes - 1), step = tm.threads >> ll;
-  for (int32_t base = 0; base < n; base += step) {
-    const int32_t q = base + (tm.id >> ll), i = r0 + q;
-    const bool valid = q < n;
-    const int32_t lo = valid ? (int32_t)__ldg(ptr + i) : 0, hi = valid ? (int32_t)__ldg(ptr + i + 1) : 0;
-    V<float, NR> s;
+      if (j[k] >= 0) v[k] = get(j[k]);
 #pragma unroll
     for (int c = 0; c < NR; ++c) s.c[c] = 0.0f;
-    for (int32_t e0 = lo + sub; e0 < hi; e0 += 8 * lanes) {
-      float a[8];
-      int32_t j[8];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const int32_t e = e0 + k * lanes;
-        const bool in = e < hi;
-        a[k] = in ? w(e) : 0.0f;
-        j[k] = in ? col(e, i) : -1;
-      }
+    for (int k = 0; k < 8; ++k)
+      if (j[k] >= 0)
+#pragma unroll
+        for (int c = 0; c < NR; ++c) s.c[c] += a[k] * v[k].c[c];
+    for (int32_t e0 = lo + at.sub + 8 * lanes; e0 < hi; e0 += 8 * lanes) {
+      entries(e0, i);
 #pragma unroll
       for (int k = 0; k < 8; ++k)
-        if (j[k] >= 0) {
-          const V<float, NR> g = get(j[k]);
+        if (j[k] >= 0) v[k] = get(j[k]);
 #pragma unroll
-          for (int c = 0; c < NR; ++c) s.c[c] += a[k] * g.c[c];
-        }
+      for (int k = 0; k < 8; ++k)
+        if (j[k] >= 0)
+#pragma unroll
+          for (int c = 0; c < NR; ++c) s.c[c] += a[k] * v[k].c[c];
     }
     for (int o = lanes >> 1; o > 0; o >>= 1)
 #pragma unroll
       for (int c = 0; c < NR; ++c) s.c[c] += __shfl_xor_sync(0xffffffffu, s.c[c], o);
-    if (sub == 0 && valid) fin(i, s);
+    if (q < at.end && at.sub == 0) fin(i, x, s);
   }
 }
-
-// log2 of the lanes per row for n rows on the team: the operator's fewest (from its row length),
-// more while threads would idle, up to eight.
-__device__ __forceinline__ int lanes_of(const Team& tm, int32_t n, int fewest) {
+// The n rows of a level over the team (alone: over its first CTA), by the operator's fewest lanes per
+// row (from its row length), more while threads would idle, up to eight.
+__device__ __forceinline__ Place place_of(const Team& tm, int32_t n, int fewest, bool alone) {
+  const int32_t threads = alone ? kTeamThreads : tm.threads;
   int ll = fewest;
-  while (ll < 3 && ((int64_t)n << (ll + 1)) <= tm.threads) ++ll;
-  return ll;
+  while (ll < 3 && ((int64_t)n << (ll + 1)) <= threads) ++ll;
+  return Place{tm.id >> ll, n, threads >> ll, tm.id & ((1 << ll) - 1), ll};
 }
 
-// One V(1,1) cycle of the chart (the launch-by-launch cycle is amg.cu vtail): lv[0].x = M^-1 lv[0].b.
-// `last` runs for each level-0 row as its value is stored; no barrier follows the last pass.
-template <int NR, class Last>
-__device__ __forceinline__ void team_vcycle(const Team& tm, const TeamShared& sh, const TeamAmg& M, int chart, int f,
-                                            Last last) {
+// The CTA's rows [r0, r1) of the system operator: in shared memory for the whole solve where they fit
+// (a step that streams it then waits for its gathers alone), else where they are.  Row offsets and
+// entries keep their global numbering.
+template <class T>
+struct OwnOp {
+  int32_t r0, r1;
+  const int32_t* rp;
+  const T* val;
+  const float* val32;  // the V-cycle's values
+  const int32_t* c32;
+  const uint16_t* c16;
+  int kind;
+  int32_t cb;
+  __device__ __forceinline__ int32_t col(int32_t e, int32_t rb) const { return kind ? rb + (int32_t)c16[e] : c32[e]; }
+  __device__ __forceinline__ int32_t base(int32_t i) const { return kind == 2 ? i - kRowRelBias : cb; }
+  template <class S, int NR, class Get>
+  __device__ __forceinline__ V<S, NR> row(const S* v, int32_t i, Get get) const {
+    const int32_t rb = base(i);
+    return entries_dot<S, NR>(
+        rp[i], rp[i + 1], [&](int32_t e) { return v[e]; }, [&](int32_t e) { return col(e, rb); }, get);
+  }
+};
+
+// One V(1,1) cycle of the chart (the launch-by-launch cycle is amg.cu vtail): lv[0].x = M^-1 lv[0].b.  The
+// pre-smoothed values w D^-1 b of level 0 are there already (in x, or y under a tentative
+// prolongator) and published; each restriction forms the next level's.  Levels of few rows (from
+// `tail` on) run on the team's first CTA between block barriers.  `last` runs for each level-0 row as
+// its value is stored; no barrier follows the last pass.
+constexpr int32_t kTeamTail = 512;
+template <int NR, class Op, class Last>
+__device__ __forceinline__ void team_vcycle(const Team& tm, const TeamShared& sh, const TeamAmg& M, const Op& op, int chart,
+                                            int f, int tail, Last last) {
   using Vf = V<float, NR>;
+  struct Early {
+    Vf a, b;
+  };
+  const bool first = tm.rank == 0;
+  // the barrier in front of a step that reads what level k's steps wrote
+  auto bar_after = [&](int k) {
+    if (k >= tail) __syncthreads();
+    else tm.bar();
+  };
   for (int k = 0; k < f; ++k) {
     const TeamLevel& L = M.lv[k];
-    const Cols cols{L.cols, L.c16, L.kind, L.kind == 1 ? __ldg(L.cbase + chart) : 0};
-    const int32_t n = sh.lvl_n[k];
-    // t = b - A (w D^-1 b), the pre-smoothed neighbours formed on the fly
-    level_rows<NR>(
-        tm, sh.lvl_row[k], n, lanes_of(tm, n, L.a_lanes), L.rp,
-        [&](int32_t e, int32_t i) { return cols.at(e, cols.base(i)); }, [&](int32_t e) { return __ldg(L.vals + e); },
-        [&](int32_t j) {
-          Vf v = ldv<float, NR>(L.b, j);
-          const float wd = kTeamOmega * __ldg(L.dinv + j);
+    const TeamLevel& C = M.lv[k + 1];
+    // t = b - A x, x the pre-smoothed values
+    const float* xp = L.smoothed ? L.x : L.y;
+    if (k == 0) {
+      for (int32_t i = op.r0 + (int32_t)threadIdx.x; i < op.r1; i += kTeamThreads) {
+        const Vf bi = ldv<float, NR>(L.b, i);
+        Vf t = op.template row<float, NR>(op.val32, i, [&](int32_t j) { return ldv<float, NR>(xp, j); });
 #pragma unroll
-          for (int c = 0; c < NR; ++c) v.c[c] *= wd;
-          return v;
-        },
-        [&](int32_t i, const Vf& s) {
-          const Vf bi = ldv<float, NR>(L.b, i);
-          Vf xi, ti;
-          const float wd = kTeamOmega * __ldg(L.dinv + i);
+        for (int c = 0; c < NR; ++c) t.c[c] = bi.c[c] - t.c[c];
+        stv<float, NR>(L.t, i, t);
+      }
+    } else if (k < tail || first) {
+      const Cols cols{L.cols, L.c16, L.kind, L.kind == 1 ? __ldg(L.cbase + chart) : 0};
+      level_step<NR>(
+          place_of(tm, sh.lvl_n[k], L.a_lanes, k >= tail), sh.lvl_row[k], L.rp,
+          [&](int32_t e, int32_t i) { return cols.at(e, cols.base(i)); }, [&](int32_t e) { return __ldg(L.vals + e); },
+          [&](int32_t j) { return ldv<float, NR>(xp, j); }, [&](int32_t i) { return ldv<float, NR>(L.b, i); },
+          [&](int32_t i, const Vf& bi, const Vf& s) {
+            Vf t;
 #pragma unroll
-          for (int c = 0; c < NR; ++c) {
-            xi.c[c] = wd * bi.c[c];
-            ti.c[c] = bi.c[c] - s.c[c];
-          }
-          if (L.smoothed) stv<float, NR>(L.x, i, xi);
-          stv<float, NR>(L.t, i, ti);
-        });
-    tm.bar();
-    // b_c = R t
-    const int32_t nc = sh.lvl_n[k + 1];
-    level_rows<NR>(
-        tm, sh.lvl_row[k + 1], nc, lanes_of(tm, nc, L.r_lanes), L.roff,
-        [&](int32_t e, int32_t) { return __ldg(L.rc + e); }, [&](int32_t e) { return __ldg(L.rv + e); },
-        [&](int32_t j) { return ldv<float, NR>(L.t, j); },
-        [&](int32_t i, const Vf& s) { stv<float, NR>(M.lv[k + 1].b, i, s); });
-    tm.bar();
+            for (int c = 0; c < NR; ++c) t.c[c] = bi.c[c] - s.c[c];
+            stv<float, NR>(L.t, i, t);
+          },
+          [&]() { bar_after(k); });
+    }
+    // b_c = R t and the coarse level's pre-smoothed values
+    float* xc = C.smoothed && k + 1 < f ? C.x : C.y;
+    if (k + 1 < tail || first) {
+      level_step<NR>(
+          place_of(tm, sh.lvl_n[k + 1], L.r_lanes, k + 1 >= tail), sh.lvl_row[k + 1], L.roff,
+          [&](int32_t e, int32_t) { return __ldg(L.rc + e); }, [&](int32_t e) { return __ldg(L.rv + e); },
+          [&](int32_t j) { return ldv<float, NR>(L.t, j); }, [&](int32_t i) { return kTeamOmega * __ldg(C.dinv + i); },
+          [&](int32_t i, float wd, const Vf& s) {
+            stv<float, NR>(C.b, i, s);
+            Vf y;
+#pragma unroll
+            for (int c = 0; c < NR; ++c) y.c[c] = wd * s.c[c];
+            stv<float, NR>(xc, i, y);
+          },
+          [&]() { bar_after(k); });
+    } else if (k < tail) {
+      tm.bar();  // (the first CTA's step has its barrier inside)
+    }
+  }
+  if (f > 0) {
+    if (f < tail) tm.bar();
+    else if (first) __syncthreads();
   }
   {  // the last level: the dense inverse (symmetric: row i read along its columns), 8 lanes a row
     const TeamLevel& L = M.lv[f];
     const int32_t r0 = sh.lvl_row[f], m = sh.lvl_n[f];
     if (m > kTeamDirect) {  // aggregation stalled above the dense limit: x = D^-1 b
-      for (int32_t i = r0 + tm.id; i < r0 + m; i += tm.threads) {
-        Vf v = ldv<float, NR>(L.b, i);
-        const float d = __ldg(L.dinv + i);
+      if (f < tail || first)
+        for (int32_t i = r0 + tm.id; i < r0 + m; i += f < tail ? tm.threads : kTeamThreads) {
+          Vf v = ldv<float, NR>(L.b, i);
+          const float d = __ldg(L.dinv + i);
 #pragma unroll
-        for (int c = 0; c < NR; ++c) v.c[c] *= d;
-        stv<float, NR>(L.x, i, v);
-        if (f == 0) last(i, v);
-      }
-    } else if (tm.rank == 0) {
+          for (int c = 0; c < NR; ++c) v.c[c] *= d;
+          stv<float, NR>(L.x, i, v);
+          if (f == 0) last(i, v);
+        }
+    } else if (first) {
       const float* Ainv = M.fac + __ldg(M.fac_off + chart);
       const int i = threadIdx.x >> 3, sub = threadIdx.x & 7;  // 64 rows x 8 lanes = one CTA
       Vf s;
@@ -429,46 +354,55 @@ __device__ __forceinline__ void team_vcycle(const Team& tm, const TeamShared& sh
     }
   }
   for (int k = f - 1; k >= 0; --k) {
-    tm.bar();
     const TeamLevel& L = M.lv[k];
     const float* xc = M.lv[k + 1].x;
-    const Cols cols{L.cols, L.c16, L.kind, L.kind == 1 ? __ldg(L.cbase + chart) : 0};
+    const bool mine = k < tail || first;
     const int32_t r0 = sh.lvl_row[k], n = sh.lvl_n[k];
-    const int la = lanes_of(tm, n, L.a_lanes);
-    auto col = [&](int32_t e, int32_t i) { return cols.at(e, cols.base(i)); };
-    auto w = [&](int32_t e) { return __ldg(L.vals + e); };
-    auto smooth = [&](auto yval) {  // x = y + w D^-1 (b - A y)
-      level_rows<NR>(tm, r0, n, la, L.rp, col, w, yval, [&](int32_t i, const Vf& s) {
-        const Vf bi = ldv<float, NR>(L.b, i), yi = yval(i);
-        Vf xi;
-        const float wd = kTeamOmega * __ldg(L.dinv + i);
-#pragma unroll
-        for (int c = 0; c < NR; ++c) xi.c[c] = yi.c[c] + wd * (bi.c[c] - s.c[c]);
-        stv<float, NR>(L.x, i, xi);
-        if (k == 0) last(i, xi);
-      });
-    };
-    if (L.smoothed) {
-      level_rows<NR>(
-          tm, r0, n, lanes_of(tm, n, L.p_lanes), L.poff, [&](int32_t e, int32_t) { return __ldg(L.pc + e); },
-          [&](int32_t e) { return __ldg(L.pv + e); }, [&](int32_t j) { return ldv<float, NR>(xc, j); },
-          [&](int32_t i, const Vf& s) {
-            Vf y = ldv<float, NR>(L.x, i);
+    // (a chain of steps on the first CTA ends with the barrier in front of the first step of all)
+    auto bar = [&]() { bar_after(k); };
+    if (L.smoothed && mine)  // y = x + P x_c
+      level_step<NR>(
+          k == 0 ? Place{op.r0 - r0 + (int32_t)threadIdx.x, op.r1 - r0, kTeamThreads, 0, 0}
+                 : place_of(tm, n, L.p_lanes, k >= tail),
+          r0, L.poff, [&](int32_t e, int32_t) { return __ldg(L.pc + e); }, [&](int32_t e) { return __ldg(L.pv + e); },
+          [&](int32_t j) { return ldv<float, NR>(xc, j); }, [&](int32_t i) { return ldv<float, NR>(L.x, i); },
+          [&](int32_t i, Vf y, const Vf& s) {
 #pragma unroll
             for (int c = 0; c < NR; ++c) y.c[c] += s.c[c];
             stv<float, NR>(L.y, i, y);
-          });
-      tm.bar();
-      smooth([&](int32_t j) { return ldv<float, NR>(L.y, j); });
-    } else {  // tentative: y_j = w D^-1_j b_j + alpha_c x_c[agg[j]] formed on the fly
-      smooth([&](int32_t j) {
-        Vf v = ldv<float, NR>(L.b, j);
-        const float wd = kTeamOmega * __ldg(L.dinv + j);
-        const Vf c = ldv<float, NR>(xc, __ldg(L.agg + j));
+          },
+          bar);
+    // x = y + w D^-1 (b - A y); a tentative prolongator's y_j is the pre-smoothed value (kept in y) plus
+    // alpha_c x_c[agg[j]], formed on the fly
+    auto yval = [&](int32_t j) {
+      Vf v = ldv<float, NR>(L.y, j);
+      if (L.smoothed) return v;
+      const Vf c = ldv<float, NR>(xc, __ldg(L.agg + j));
 #pragma unroll
-        for (int q = 0; q < NR; ++q) v.c[q] = wd * v.c[q] + M.alpha_c * c.c[q];
-        return v;
-      });
+      for (int q = 0; q < NR; ++q) v.c[q] += M.alpha_c * c.c[q];
+      return v;
+    };
+    auto early = [&](int32_t i) { return Early{ldv<float, NR>(L.b, i), yval(i)}; };
+    auto fin = [&](int32_t i, const Early& x, const Vf& s) {
+      const float wd = kTeamOmega * __ldg(L.dinv + i);
+      Vf z;
+#pragma unroll
+      for (int c = 0; c < NR; ++c) z.c[c] = x.b.c[c] + wd * (x.a.c[c] - s.c[c]);
+      stv<float, NR>(L.x, i, z);
+      if (k == 0) last(i, z);
+    };
+    if (k == 0) {
+      tm.bar();
+      for (int32_t i = op.r0 + (int32_t)threadIdx.x; i < op.r1; i += kTeamThreads) {
+        const Early x = early(i);
+        fin(i, x, op.template row<float, NR>(op.val32, i, yval));
+      }
+    } else if (mine) {
+      const Cols cols{L.cols, L.c16, L.kind, L.kind == 1 ? __ldg(L.cbase + chart) : 0};
+      level_step<NR>(
+          place_of(tm, n, L.a_lanes, k >= tail), r0, L.rp,
+          [&](int32_t e, int32_t i) { return cols.at(e, cols.base(i)); }, [&](int32_t e) { return __ldg(L.vals + e); }, yval,
+          early, fin, bar);
     }
   }
 }
@@ -550,12 +484,19 @@ struct TeamSys {
   const uint16_t* c16;
   const int32_t* cbase;
   int kind;
-  const float* vals32;
+  int store_bytes;  // dynamic shared memory for a CTA's rows of the operator
 };
+
+// CTAs on an SM: the FP32 loop without a preconditioner of its own fits 64 registers a thread; the others
+// take 128 (spilled values would come back from L2, past an L1 that every cluster barrier empties).
+template <class S, int PCK>
+constexpr int team_per_sm() {
+  return std::is_same<S, float>::value && PCK == 0 ? 2 : 1;
+}
 
 // PCK: 0 none or Jacobi, 1 AMG, 2 IC(0).
 template <class S, int NR, int PCK>
-__global__ void __launch_bounds__(kTeamThreads, std::is_same<S, double>::value ? 1 : 2)
+__global__ void __launch_bounds__(kTeamThreads, team_per_sm<S, PCK>())
     k_team(const __grid_constant__ TeamSys A, const __grid_constant__ TeamLoop<S> P,
            const __grid_constant__ TeamAmg M, const __grid_constant__ TeamIc0 I) {
   constexpr bool mixed = std::is_same<S, float>::value;
@@ -587,8 +528,38 @@ __global__ void __launch_bounds__(kTeamThreads, std::is_same<S, double>::value ?
   if (sh.st.state != kActive) return;  // (the whole team)
   if (tm.ctas > 1) tm.bar();           // the whole team runs before anyone writes a peer's memory
   const int32_t r0 = (int32_t)A.chart_row[chart], r1 = (int32_t)A.chart_row[chart + 1];
-  const Cols cols{A.cols, A.c16, A.kind, A.kind == 1 ? A.cbase[chart] : 0};
-  int f = 0;
+  // this CTA's rows, and their part of the operator
+  constexpr bool copies = PCK == 1 && !mixed;  // FP32 cycle under the FP64 loop
+  const int32_t R0 = r0 + (int32_t)((int64_t)(r1 - r0) * tm.rank / tm.ctas);
+  const int32_t R1 = r0 + (int32_t)((int64_t)(r1 - r0) * (tm.rank + 1) / tm.ctas);
+  OwnOp<S> op{R0, R1, A.rp, P.vals, PCK == 1 ? M.lv[0].vals : nullptr, A.cols, A.c16, A.kind,
+              A.kind == 1 ? A.cbase[chart] : 0};
+  {
+    extern __shared__ __align__(16) unsigned char store[];
+    const int32_t e0 = A.rp[R0], ne = A.rp[R1] - e0;
+    const int64_t need = (int64_t)ne * (int)(sizeof(S) + (copies ? 4 : 0) + (A.kind ? 2 : 4)) + 4 * (int64_t)(R1 - R0 + 1);
+    if (need <= (int64_t)A.store_bytes) {
+      S* v = reinterpret_cast<S*>(store);
+      float* v32 = reinterpret_cast<float*>(v + ne);
+      int32_t* rp = reinterpret_cast<int32_t*>(v32 + (copies ? ne : 0));
+      int32_t* c32 = rp + (R1 - R0 + 1);
+      uint16_t* c16 = reinterpret_cast<uint16_t*>(c32);
+      for (int32_t k = threadIdx.x; k <= R1 - R0; k += kTeamThreads) rp[k] = A.rp[R0 + k];
+      for (int32_t k = threadIdx.x; k < ne; k += kTeamThreads) {
+        v[k] = P.vals[e0 + k];
+        if (copies) v32[k] = M.lv[0].vals[e0 + k];
+        if (A.kind) c16[k] = A.c16[e0 + k];
+        else c32[k] = A.cols[e0 + k];
+      }
+      __syncthreads();
+      op.rp = rp - R0;
+      op.val = v - e0;
+      op.val32 = copies ? v32 - e0 : reinterpret_cast<const float*>(v) - e0;
+      op.c32 = c32 - e0;
+      op.c16 = c16 - e0;
+    }
+  }
+  int f = 0, tail = kTeamMaxLevels;
   if constexpr (PCK == 1) {
     f = M.final_lvl[chart];
     if ((int)threadIdx.x <= f) {
@@ -597,8 +568,23 @@ __global__ void __launch_bounds__(kTeamThreads, std::is_same<S, double>::value ?
       sh.lvl_n[threadIdx.x] = (int32_t)(b - a);
     }
     __syncthreads();
+    for (int k = f; k > 0; --k)
+      if (sh.lvl_n[k] <= kTeamTail) tail = k;
   }
-  constexpr bool copies = PCK == 1 && !mixed;  // FP32 cycle under the FP64 loop
+  // a row's r has its final value for the V-cycle: level 0's right-hand side and pre-smoothed values
+  auto put_r = [&](int32_t i, const Vs& r) {
+    if constexpr (PCK == 1) {
+      const float wd = kTeamOmega * __ldg(M.lv[0].dinv + i);
+      V<float, NR> t, x;
+#pragma unroll
+      for (int c = 0; c < NR; ++c) {
+        t.c[c] = (float)r.c[c];
+        x.c[c] = wd * t.c[c];
+      }
+      if (copies) stv<float, NR>(P.r32, i, t);
+      stv<float, NR>(M.lv[0].smoothed ? M.lv[0].x : M.lv[0].y, i, x);
+    }
+  };
 
   // z = M^-1 r and the sums r.z, z.q of a separate preconditioner, then fn
   auto apply = [&](auto fn) -> int {
@@ -612,7 +598,7 @@ __global__ void __launch_bounds__(kTeamThreads, std::is_same<S, double>::value ?
       }
     };
     if constexpr (PCK == 1) {
-      team_vcycle<NR>(tm, sh, M, chart, f, [&](int32_t i, const V<float, NR>& z) {
+      team_vcycle<NR>(tm, sh, M, op, chart, f, tail, [&](int32_t i, const V<float, NR>& z) {
         Vs zv;
 #pragma unroll
         for (int c = 0; c < NR; ++c) zv.c[c] = (S)z.c[c];
@@ -634,7 +620,7 @@ __global__ void __launch_bounds__(kTeamThreads, std::is_same<S, double>::value ?
             stv<S, NR>(zp, i, v);
             if (to) stv<S, NR>(P.z, __ldg(to + i), v);
           });
-      for (int32_t i = r0 + tm.id; i < r1; i += tm.threads) dots(i, ldv<S, NR>(P.z, i));
+      for (int32_t i = R0 + (int32_t)threadIdx.x; i < R1; i += kTeamThreads) dots(i, ldv<S, NR>(P.z, i));
     }
     const int flag = team_reduce<2, S>(tm, sh, acc, fn);
     if (PCK == 1) tm.publish();  // z (the sweeps' last barrier has published theirs)
@@ -659,29 +645,22 @@ __global__ void __launch_bounds__(kTeamThreads, std::is_same<S, double>::value ?
 
   int flag = kGo;
   if constexpr (PCK != 0) {
-    if constexpr (copies) {
-      for (int32_t i = r0 + tm.id; i < r1; i += tm.threads) {
-        const Vs r = ldv<S, NR>(P.r, i);
-        V<float, NR> t;
-#pragma unroll
-        for (int c = 0; c < NR; ++c) t.c[c] = (float)r.c[c];
-        stv<float, NR>(P.r32, i, t);
-      }
-    }
+    if constexpr (PCK == 1)
+      for (int32_t i = R0 + (int32_t)threadIdx.x; i < R1; i += kTeamThreads) put_r(i, ldv<S, NR>(P.r, i));
     tm.bar();
     flag = apply([&](const Sc (&t)[2]) {
       sh.s_rz = sc_bits(t[0]);
       return (int)kGo;
     });
-    for (int32_t i = r0 + tm.id; i < r1; i += tm.threads) stv<S, NR>(P.p, i, zrow(i));
+    for (int32_t i = R0 + (int32_t)threadIdx.x; i < R1; i += kTeamThreads) stv<S, NR>(P.p, i, zrow(i));
     tm.bar();
   }
   while (flag < kStop) {
     // q = A p, p.q
     S pq[1] = {S(0)};
-    for (int32_t i = r0 + tm.id; i < r1; i += tm.threads) {
-      const Vs s = row_dot<S, NR>(A.rp, cols, P.vals, i, [&](int32_t j) { return ldv<S, NR>(P.p, j); });
+    for (int32_t i = R0 + (int32_t)threadIdx.x; i < R1; i += kTeamThreads) {
       const Vs pi = ldv<S, NR>(P.p, i);
+      const Vs s = op.template row<S, NR>(op.val, i, [&](int32_t j) { return ldv<S, NR>(P.p, j); });
       stv<S, NR>(P.q, i, s);
 #pragma unroll
       for (int c = 0; c < NR; ++c) pq[0] += pi.c[c] * s.c[c];
@@ -701,7 +680,7 @@ __global__ void __launch_bounds__(kTeamThreads, std::is_same<S, double>::value ?
     // x += alpha p, r -= alpha q; r.r and (plain loop) r.z
     const S alpha = mixed ? (S)sh.alpha32 : (S)sh.alpha;
     S rr[2] = {S(0), S(0)};
-    for (int32_t i = r0 + tm.id; i < r1; i += tm.threads) {
+    for (int32_t i = R0 + (int32_t)threadIdx.x; i < R1; i += kTeamThreads) {
       Vs xv = ldv<S, NR>(P.x, i), rv = ldv<S, NR>(P.r, i);
       const Vs pv = ldv<S, NR>(P.p, i), qv = ldv<S, NR>(P.q, i);
       const S di = PCK == 0 && P.jacobi ? __ldg(P.dinv + i) : S(1);
@@ -714,12 +693,7 @@ __global__ void __launch_bounds__(kTeamThreads, std::is_same<S, double>::value ?
       }
       stv<S, NR>(P.x, i, xv);
       stv<S, NR>(P.r, i, rv);
-      if constexpr (copies) {
-        V<float, NR> t;
-#pragma unroll
-        for (int c = 0; c < NR; ++c) t.c[c] = (float)rv.c[c];
-        stv<float, NR>(P.r32, i, t);
-      }
+      put_r(i, rv);
     }
     auto new_beta = [&](Sc rznew) {
       const Sc beta = sc_div(rznew, sc_of_bits(Sc{}, sh.s_rz));
@@ -760,7 +734,7 @@ __global__ void __launch_bounds__(kTeamThreads, std::is_same<S, double>::value ?
         fresh = true;
         // fold the FP32 increment into the double-float solution, then r = b - A x (pcg.cu
         // k_fold, k_true_residual)
-        for (int32_t i = r0 + tm.id; i < r1; i += tm.threads) {
+        for (int32_t i = R0 + (int32_t)threadIdx.x; i < R1; i += kTeamThreads) {
           DF<NR> xv = lddf<NR>(P.xdf, i);
           const V<float, NR> dv = ldv<float, NR>(P.x, i);
           V<float, NR> zero;
@@ -779,23 +753,32 @@ __global__ void __launch_bounds__(kTeamThreads, std::is_same<S, double>::value ?
         tm.bar();
         const float rsc = sh.st.rscale;
         float acc[2] = {0.0f, 0.0f};
-        for (int32_t i = r0 + tm.id; i < r1; i += tm.threads) {
-          const int32_t lo = __ldg(A.rp + i), hi = __ldg(A.rp + i + 1), rb = cols.base(i);
+        for (int32_t i = R0 + (int32_t)threadIdx.x; i < R1; i += kTeamThreads) {
+          const int32_t lo = op.rp[i], hi = op.rp[i + 1], rb = op.base(i);
           const DF<NR> xi = lddf<NR>(P.xdf, i);
           float Sh[NR], Sl[NR];
 #pragma unroll
           for (int c = 0; c < NR; ++c) Sh[c] = Sl[c] = 0.0f;
-#pragma unroll 4
-          for (int32_t e = lo; e < hi; ++e) {
-            const float ah = __ldg(P.vals + e), al = __ldg(P.vals_lo + e);
-            const DF<NR> xj = lddf<NR>(P.xdf, cols.at(e, rb));
+          for (int32_t e0 = lo; e0 < hi; e0 += 4) {  // four neighbours in flight
+            float ah[4], al[4];
+            DF<NR> xj[4];
 #pragma unroll
-            for (int c = 0; c < NR; ++c) {
-              float dh, dl;
-              two_sum(xj.h[c], -xi.h[c], dh, dl);
-              dl += xj.l[c] - xi.l[c];
-              df_fma(ah, al, dh, dl, Sh[c], Sl[c]);
-            }
+            for (int q = 0; q < 4; ++q)
+              if (e0 + q < hi) {
+                ah[q] = (float)op.val[e0 + q];
+                al[q] = __ldg(P.vals_lo + e0 + q);
+                xj[q] = lddf<NR>(P.xdf, op.col(e0 + q, rb));
+              }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              if (e0 + q < hi)
+#pragma unroll
+                for (int c = 0; c < NR; ++c) {
+                  float dh, dl;
+                  two_sum(xj[q].h[c], -xi.h[c], dh, dl);
+                  dl += xj[q].l[c] - xi.l[c];
+                  df_fma(ah[q], al[q], dh, dl, Sh[c], Sl[c]);
+                }
           }
           const float2 rs = __ldg(P.rsum + i);
           const DF<NR> bv = lddf<NR>(P.bdf, i);
@@ -817,6 +800,7 @@ __global__ void __launch_bounds__(kTeamThreads, std::is_same<S, double>::value ?
             acc[1] += t * (rv.c[c] * di * rsc);
           }
           stv<float, NR>(P.r, i, rv);
+          put_r(i, rv);
         }
         flag = team_reduce<2, float>(tm, sh, acc, [&](const Pair (&t)[2]) {
           const double inv = 1.0 / ((double)rsc * (double)rsc);
@@ -860,7 +844,7 @@ __global__ void __launch_bounds__(kTeamThreads, std::is_same<S, double>::value ?
     }
     // p = z + beta p
     const S beta = mixed ? (S)sh.beta32 : (S)sh.beta;
-    for (int32_t i = r0 + tm.id; i < r1; i += tm.threads) {
+    for (int32_t i = R0 + (int32_t)threadIdx.x; i < R1; i += kTeamThreads) {
       const Vs zv = zrow(i);
       Vs pv = ldv<S, NR>(P.p, i);
 #pragma unroll
@@ -870,7 +854,7 @@ __global__ void __launch_bounds__(kTeamThreads, std::is_same<S, double>::value ?
     tm.bar();
   }
   if constexpr (mixed) {  // fold what is pending; the FP64 solution is hi + lo
-    for (int32_t i = r0 + tm.id; i < r1; i += tm.threads) {
+    for (int32_t i = R0 + (int32_t)threadIdx.x; i < R1; i += kTeamThreads) {
       DF<NR> xv = lddf<NR>(P.xdf, i);
       const V<float, NR> dv = ldv<float, NR>(P.x, i);
       V<float, NR> zero;
@@ -901,27 +885,35 @@ __global__ void __launch_bounds__(kTeamThreads, std::is_same<S, double>::value ?
 }
 
 // ---------------------------------------------------------------- which charts, and how many CTAs
-// CTAs of a chart's team (0: left to the launch-per-step loop).
-int team_size(int64_t rows, bool mixed, int kind, int64_t width) {
-  // one CTA while a step fits it: its block barrier costs tens of clocks, a cluster's over a
-  // thousand; FP64 rows are bound by the SM's FP64 pipe instead and spread out earlier
-  const int64_t per = mixed ? 1024 : 256;
-  int64_t want = (rows + per - 1) / per;
-  if (kind == 2) want = std::max<int64_t>(1, width / 256);
-  const int64_t lim = mixed ? 131072 : 40000;
-  if (rows > lim) return 0;
+constexpr int64_t kTeamAmgRows = 600000;
+// CTAs of a team for `want` CTAs' worth of work.
+int team_ctas(int64_t want) {
   int c = 1;
   while (c < want && c < kTeamMaxCtas) c *= 2;
   return c;
 }
 
+// Bytes of a row of the operator in shared memory.
+template <class S, int PCK>
+double store_row(double per_row, bool narrow) {
+  return per_row * (double)(sizeof(S) + (PCK == 1 && sizeof(S) == 8 ? 4 : 0) + (narrow ? 2 : 4)) + 4.0;
+}
+
 template <class S, int NR, int PCK>
-void launch_team(cudaStream_t s, int ctas, int64_t n, const TeamSys& A, const TeamLoop<S>& P, const TeamPrecond* pc) {
+void launch_team(cudaStream_t s, int ctas, int64_t n, int64_t rows, double per_row, TeamSys A, const TeamLoop<S>& P,
+                 const TeamPrecond* pc) {
   auto k = k_team<S, NR, PCK>;
+  // room for the largest chart's share of the operator (a CTA with more reads it from global memory),
+  // as long as the CTAs that the registers allow on an SM still fit
+  const int64_t want = (int64_t)(1.1 * store_row<S, PCK>(per_row, A.kind != 0) * (double)((rows + ctas - 1) / ctas)) + 1024;
+  const int64_t most = (team_per_sm<S, PCK>() == 2 ? 104 : 200) * 1024;
+  A.store_bytes = want <= most ? (int)((want + 15) & ~(int64_t)15) : 0;
+  RUV_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
   if (ctas > 8) RUV_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(n * ctas));
   cfg.blockDim = dim3(kTeamThreads);
+  cfg.dynamicSmemBytes = (size_t)A.store_bytes;
   cfg.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -937,6 +929,11 @@ void launch_team(cudaStream_t s, int ctas, int64_t n, const TeamSys& A, const Te
 
 }  // namespace
 
+bool teams_on(const Ctx& ctx) {
+  const char* e = std::getenv("RUV_TEAM");
+  return !((e && e[0] == '0') || std::getenv("RUV_SPMV_TMA") || std::getenv("RUV_AMG_STAGE") || ctx.shape_forced);
+}
+
 void Ctx::team_streams(int n) {
   if (!team_go) RUV_CUDA(cudaEventCreateWithFlags(&team_go, cudaEventDisableTiming));
   for (int k = 0; k < n; ++k) {
@@ -948,26 +945,45 @@ void Ctx::team_streams(int n) {
 template <class S, int NR>
 int64_t team_solve(Ctx& ctx, const DevSystem& sys, const TeamLoop<S>& loop, const TeamPrecond* pc) {
   const int64_t NC = sys.n_charts;
-  // RUV_TEAM=0, or a knob that picks a kernel of the launch-per-step loop: that loop for all
-  const char* e = std::getenv("RUV_TEAM");
-  const bool off = (e && e[0] == '0') || std::getenv("RUV_SPMV_TMA") || std::getenv("RUV_AMG_STAGE") || ctx.shape_forced;
   const int kind = pc ? pc->kind : 0;
+  constexpr bool mixed = std::is_same<S, float>::value;
+  auto rows_of = [&](int64_t c) { return sys.h_chart_row[c + 1] - sys.h_chart_row[c]; };
   int64_t left = 0, largest = 0;
-  for (int64_t c = 0; c < NC; ++c) largest = std::max(largest, sys.h_chart_row[c + 1] - sys.h_chart_row[c]);
-  // a V-cycle is a chain of a dozen small steps: by teams only where one CTA holds every chart
-  const bool none = off || (pc && kind == 0) || (kind == 1 && largest > 1024);
+  for (int64_t c = 0; c < NC; ++c) largest = std::max(largest, rows_of(c));
+  const char* re = std::getenv("RUV_TEAM_ROWS");
+  const int64_t most = re ? std::atoll(re) : mixed ? 131072 : 40000;
+  // a V-cycle is a chain of small steps, and a chart left to the other loop makes them all again: all
+  // charts by teams, or none.  Teams hold 512 rows in flight on an SM where the launch loop's kernels
+  // stream: 473,000 rows in 300 charts took 146 us an iteration against 172, 14.4 million 7,000 against
+  // 2,900.
+  const bool none = !teams_on(ctx) || (pc && kind == 0) ||
+                    (kind == 1 && (largest > most || sys.n_rows > kTeamAmgRows));
+  // Rows per CTA: as few as let every team run at once.  An FP32 step of one CTA of 512 threads costs
+  // little more for two rows a thread, and its block barrier tens of clocks where a cluster's takes
+  // over a thousand; FP64 rows are bound by the SM's FP64 pipe and spread out earlier.
+  const char* pe = std::getenv("RUV_TEAM_PER");
+  int64_t per = mixed ? (kind == 1 ? 512 : 1024) : 256;
+  const int64_t slots = (mixed && kind == 0 ? 2 : 1) * (int64_t)ctx.sm_count, per_most = mixed ? 2048 : 1024;
+  if (pe) {
+    per = std::max(64, std::atoi(pe));
+  } else if (kind != 2) {
+    for (; per < per_most; per *= 2) {
+      int64_t ctas = 0;
+      for (int64_t c = 0; c < NC; ++c) ctas += rows_of(c) > 0 ? team_ctas((rows_of(c) + per - 1) / per) : 0;
+      if (ctas <= slots) break;
+    }
+  }
   // charts by team size, the largest first within each
   std::vector<int32_t> cls[5];
   for (int64_t c = 0; c < NC; ++c) {
-    const int64_t rows = sys.h_chart_row[c + 1] - sys.h_chart_row[c];
+    const int64_t rows = rows_of(c);
     if (rows == 0) continue;
-    const int ctas = none ? 0
-                     : team_size(rows, std::is_same<S, float>::value, kind, pc && kind == 2 ? pc->ic0.width : 0);
-    if (ctas == 0) {
+    if (none || rows > most) {
       ++left;
       continue;
     }
-    cls[__builtin_ctz(ctas)].push_back((int32_t)c);
+    const int64_t want = kind == 2 ? std::max<int64_t>(1, pc->ic0.width / 256) : (rows + per - 1) / per;
+    cls[__builtin_ctz(team_ctas(want))].push_back((int32_t)c);
   }
   std::vector<int32_t> order;
   int64_t first[6] = {0};
@@ -1009,10 +1025,12 @@ int64_t team_solve(Ctx& ctx, const DevSystem& sys, const TeamLoop<S>& loop, cons
     const int64_t n = first[k + 1] - first[k];
     if (n == 0) continue;
     cudaStream_t s = --classes == 0 ? main : ctx.team_stream[join.used++];
-    const TeamSys A{d_order + first[k], sys.chart_row, sys.row_ptr, sys.cols, sys.cols16, sys.cbase, nw, sys.vals32};
-    if (kind == 1) launch_team<S, NR, 1>(s, 1 << k, n, A, loop, pc);
-    else if (kind == 2) launch_team<S, NR, 2>(s, 1 << k, n, A, loop, pc);
-    else launch_team<S, NR, 0>(s, 1 << k, n, A, loop, pc);
+    const TeamSys A{d_order + first[k], sys.chart_row, sys.row_ptr, sys.cols, sys.cols16, sys.cbase, nw, 0};
+    const int64_t rows = rows_of(order[first[k]]);  // the class's largest
+    const double per_row = (double)sys.nnz / (double)sys.n_rows;
+    if (kind == 1) launch_team<S, NR, 1>(s, 1 << k, n, rows, per_row, A, loop, pc);
+    else if (kind == 2) launch_team<S, NR, 2>(s, 1 << k, n, rows, per_row, A, loop, pc);
+    else launch_team<S, NR, 0>(s, 1 << k, n, rows, per_row, A, loop, pc);
   }
   RUV_LAUNCH_CHECK();
   return left;

@@ -70,8 +70,12 @@ struct TeamLoop {
   int jacobi;  // plain loop: 1 Jacobi, 0 none
 };
 
-// Solves every chart a team is the faster way for and marks it done in loop.st; returns the
-// number of charts left to the launch-per-step loop.
+// Whether the kernels below may be used: not under RUV_TEAM=0 or a knob that picks a kernel of the
+// launch-per-step loop (RUV_LPR, RUV_SPMV_TMA, RUV_AMG_STAGE).
+bool teams_on(const Ctx& ctx);
+
+// Solves every chart that a team is the faster way for and marks it done in loop.st; returns the
+// number of charts left.
 template <class S, int NR>
 int64_t team_solve(Ctx& ctx, const DevSystem& sys, const TeamLoop<S>& loop, const TeamPrecond* pc);
 

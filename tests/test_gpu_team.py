@@ -47,7 +47,7 @@ SIZES = [(3, 3), (33, 3), (34, 3), (18, 34), (34, 34), (35, 34), (66, 34), (67, 
                                      R.Precond.IC0_COLOR])
 def test_team_matches_launch_loop(monkeypatch, precond, precision):
     vo, to, p3, tr = [0], [0], [], []
-    for nx, ny in SIZES if precond not in (R.Precond.AMG, R.Precond.AMG_SA) else SIZES[:5]:
+    for nx, ny in SIZES:
         p, f = _grid(nx, ny)
         p3.append(p)
         tr.append(f)
