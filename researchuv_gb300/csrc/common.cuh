@@ -181,6 +181,22 @@ __device__ __forceinline__ void block_sum_t(A (&v)[NV], A* sh) {
   __syncthreads();
 }
 
+// The same totals in thread 0 alone, for one use of `sh` in a kernel: the last step runs in one warp (in
+// FP64 every warp that repeats it costs the SM's FP64 pipe 100 clocks a value).
+template <int NV, class A>
+__device__ __forceinline__ void block_sum_first(A (&v)[NV], A* sh) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) v[k] = warp_sum(v[k]);
+  if (lane == 0)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) sh[k * 32 + wid] = v[k];
+  __syncthreads();
+  if (wid == 0)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] = warp_sum(lane < nw ? sh[k * 32 + lane] : A(0));
+}
+
 template <int NV>
 __device__ __forceinline__ void block_sum(double (&v)[NV], double* sh) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;

@@ -62,6 +62,142 @@ struct Tiles {
   int64_t spin_limit = 0;
 };
 
+// ---------------------------------------------------------------- chart steps
+// What follows a tile kernel's partial sums, once per chart: alpha, beta, convergence.  The last of a
+// chart's tiles to arrive does it (every tile's sum is in global memory by then), combining the
+// partials in tile order as k_chart_step does -- the same bits whichever tile is last,
+// without a kernel of its own between the tile kernels (4 to 9 us each, five an iteration).
+enum : int { kStepNone = 0, kStepAlpha, kStepBeta, kStepBetaMixed, kStepAfterRefresh, kStepCheck64, kStepRz0, kStepBetaPc };
+struct ChartStep {
+  int kind = kStepNone;
+  int precond_none = 0;  // rz is r.r
+  int separate = 0;      // the preconditioner is applied by its own launches: beta comes after it
+  int flexible = 0;
+  int64_t max_iter = 0;
+  double delta = 0.0;
+  ChartState* st = nullptr;
+  int* n_active = nullptr;
+  int32_t* done = nullptr;  // the separate preconditioner's mask
+  int32_t* arrived = nullptr;  // tiles of each chart that have their sums in place (zero between kernels)
+};
+
+__device__ __forceinline__ void chart_over(ChartState& s, const ChartStep& F, int64_t c, int status) {
+  s.status = status;
+  s.state = kDone;
+  if (F.done) F.done[c] = 1;
+  atomicSub(F.n_active, 1);
+}
+
+// One lane: the step from the chart's sums v.
+__device__ __forceinline__ void chart_step(const ChartStep& F, int64_t c, double v0, double v1) {
+  ChartState& s = F.st[c];
+  auto plain_beta = [&](double rznew) {
+    s.beta = rznew / s.rz;
+    s.beta32 = (float)s.beta;
+    s.rz = rznew;
+  };
+  switch (F.kind) {
+    case kStepAlpha:
+      if (fabs(v0) <= 1e-300 || !isfinite(v0)) return chart_over(s, F, c, RUV_ERR_BREAKDOWN);  // solver.rs:505-508
+      s.alpha = s.rz / v0;
+      s.alpha32 = (float)s.alpha;
+      break;
+    case kStepBeta:  // FP64: convergence on the recurrence residual (solver.rs:518-522), then beta
+      s.iters += 1;
+      s.rr = v0;
+      if (sqrt(v0) <= s.tol_abs) return chart_over(s, F, c, RUV_OK);
+      if (s.iters >= F.max_iter) return chart_over(s, F, c, RUV_ERR_NOT_CONVERGED);
+      plain_beta(F.precond_none ? v0 : v1);
+      break;
+    case kStepCheck64:  // the same with a separate preconditioner
+      s.iters += 1;
+      s.rr = v0;
+      if (sqrt(v0) <= s.tol_abs) return chart_over(s, F, c, RUV_OK);
+      if (!isfinite(v0)) return chart_over(s, F, c, RUV_ERR_BREAKDOWN);
+      if (s.iters >= F.max_iter) return chart_over(s, F, c, RUV_ERR_NOT_CONVERGED);
+      break;
+    case kStepBetaMixed: {  // mixed: the FP32 residual only schedules true-residual refreshes
+      s.iters += 1;
+      const double rn = sqrt(v0);
+      if (rn <= F.delta * s.r_ref || rn <= s.tol_abs || !isfinite(rn) || s.iters >= F.max_iter) {
+        s.refresh = 1;  // beta is formed after the refresh, from the true residual
+      } else {
+        s.refresh = 0;
+        if (!F.separate) plain_beta(F.precond_none ? v0 : v1);
+      }
+      break;
+    }
+    case kStepAfterRefresh: {
+      s.refinements += 1;
+      s.rr = v0;
+      const double rn = sqrt(v0);
+      if (rn <= s.tol_abs) return chart_over(s, F, c, RUV_OK);
+      if (!isfinite(rn)) return chart_over(s, F, c, RUV_ERR_BREAKDOWN);
+      if (s.iters >= F.max_iter) return chart_over(s, F, c, RUV_ERR_NOT_CONVERGED);
+      s.r_ref = rn;
+      if (F.separate) {
+        s.refresh = 2;  // refreshed: beta is the plain Fletcher-Reeves ratio
+        break;
+      }
+      plain_beta(F.precond_none ? v0 : v1);
+      s.refresh = 0;
+      break;
+    }
+    case kStepRz0:
+      s.rz = v0;
+      break;
+    case kStepBetaPc: {
+      // after a separate apply: flexible (Polak-Ribiere, as the reference's FCG for AMG,
+      // solver.rs:474-481, :526-539) using r_new - r_old = -alpha q, or Fletcher-Reeves right
+      // after a true-residual refresh (r jumped)
+      double beta = (F.flexible && s.refresh != 2) ? (-s.alpha * v1) / s.rz : v0 / s.rz;
+      if (!isfinite(beta)) beta = 0.0;
+      s.beta = beta;
+      s.beta32 = (float)beta;
+      s.rz = v0;
+      s.refresh = 0;
+      break;
+    }
+    default: break;
+  }
+}
+
+// A tile's end: its sums v (thread 0's) into part, and the chart's step by the last tile.
+template <int NV>
+__device__ __forceinline__ void tile_end(const Tiles& T, const ChartStep& F, int64_t t, int32_t ch, const double (&v)[NV],
+                                         double* part) {
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) part[NV * t + k] = v[k];
+  if (F.kind == kStepNone) return;
+  const int64_t t0 = T.chart_tile[ch], n = T.chart_tile[ch + 1] - t0;
+  if (n == 1) {
+    if (threadIdx.x == 0) chart_step(F, ch, v[0], NV > 1 ? v[NV - 1] : 0.0);
+    return;
+  }
+  __shared__ int last;
+  __shared__ double sh[NV * 32];
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(&F.arrived[ch], 1) == (int)n - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double w[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) w[k] = 0.0;
+  if (threadIdx.x < kChartThreads)
+    for (int64_t q = t0 + threadIdx.x; q < t0 + n; q += kChartThreads)
+#pragma unroll
+      for (int k = 0; k < NV; ++k) w[k] += __ldcg(part + NV * q + k);
+  block_sum_first<NV>(w, sh);
+  if (threadIdx.x == 0) {
+    F.arrived[ch] = 0;
+    chart_step(F, ch, w[0], NV > 1 ? w[NV - 1] : 0.0);
+  }
+}
+
 // ---------------------------------------------------------------- tile kernels
 // Accumulator type of the per-element loops: float in the FP32 solver (GB300's FP64 pipe is
 // a small fraction of its FP32 rate, so FP64 appears only per tile and per chart), double in
@@ -210,7 +346,7 @@ __global__ void __launch_bounds__(kTileThreads) k_spmv_pq_k(Tiles T, const Chart
                                                             const uint16_t* __restrict__ c16,
                                                             const int32_t* __restrict__ cbase, const S* __restrict__ vals,
                                                             const S* __restrict__ p, S* __restrict__ q,
-                                                            double* __restrict__ part) {
+                                                            double* __restrict__ part, ChartStep F) {
   __shared__ S sh[32];
   const int64_t t = blockIdx.x;
   const int32_t ch = T.chart[t];
@@ -220,8 +356,9 @@ __global__ void __launch_bounds__(kTileThreads) k_spmv_pq_k(Tiles T, const Chart
   if constexpr (NW == 1) spmv_pq_tile<S, NR, LPR, U>(beg, end, row_ptr, ColsNarrow{c16, cbase[ch]}, vals, p, q, acc);
   else if constexpr (NW == 2) spmv_pq_tile<S, NR, LPR, U>(beg, end, row_ptr, ColsRowRel{c16}, vals, p, q, acc);
   else spmv_pq_tile<S, NR, LPR, U>(beg, end, row_ptr, ColsWide{cols}, vals, p, q, acc);
-  block_sum_t<1, S>(acc, sh);
-  if (threadIdx.x == 0) part[t] = (double)acc[0];
+  block_sum_first<1, S>(acc, sh);
+  const double v[1] = {(double)acc[0]};
+  tile_end<1>(T, F, t, ch, v, part);
 }
 
 // ---------------------------------------------------------------- bulk-copy SpMV
@@ -369,7 +506,7 @@ __global__ void __launch_bounds__(kTileThreads) k_spmv_tma(Tiles T, const ChartS
                                                            const uint16_t* __restrict__ c16,
                                                            const int32_t* __restrict__ cbase, const S* __restrict__ vals,
                                                            const S* __restrict__ p, S* __restrict__ q,
-                                                           double* __restrict__ part) {
+                                                           double* __restrict__ part, ChartStep F) {
   extern __shared__ __align__(16) unsigned char stage[];
   __shared__ S sh[32];
   const int64_t t = blockIdx.x;
@@ -394,8 +531,9 @@ __global__ void __launch_bounds__(kTileThreads) k_spmv_tma(Tiles T, const ChartS
   S acc = S(0);
   spmv_staged_tile<S, NR, LPR, U, NW>(beg, end, w, buf, NW == 1 ? cbase[ch] : 0, p, q, acc);
   S accv[1] = {acc};
-  block_sum_t<1, S>(accv, sh);
-  if (threadIdx.x == 0) part[t] = (double)accv[0];
+  block_sum_first<1, S>(accv, sh);
+  const double v[1] = {(double)accv[0]};
+  tile_end<1>(T, F, t, ch, v, part);
 }
 
 // One launch of the SpMV for a column stream of kind nw (0 wide, 1 chart-relative, 2 row-
@@ -404,25 +542,25 @@ __global__ void __launch_bounds__(kTileThreads) k_spmv_tma(Tiles T, const ChartS
 template <class S, int NR, int LPR, int U, int NW>
 void launch_spmv_nw(cudaStream_t s, unsigned grid, const Tiles& T, const ChartState* st, const int32_t* row_ptr,
                     const int32_t* cols, const uint16_t* c16, const int32_t* cbase, const S* vals, const S* p, S* q,
-                    double* part) {
+                    double* part, const ChartStep& F) {
   if constexpr (std::is_same<S, float>::value && NR == 2) {
     const size_t sm = spmv_tma_smem<S, NW>(T);
     if (T.max_rows > 0 && sm <= kSpmvTmaMaxSmem) {
-      k_spmv_tma<S, NR, LPR, U, NW><<<grid, kTileThreads, sm, s>>>(T, st, row_ptr, cols, c16, cbase, vals, p, q, part);
+      k_spmv_tma<S, NR, LPR, U, NW><<<grid, kTileThreads, sm, s>>>(T, st, row_ptr, cols, c16, cbase, vals, p, q, part, F);
       return;
     }
   }
-  k_spmv_pq_k<S, NR, LPR, U, NW><<<grid, kTileThreads, 0, s>>>(T, st, row_ptr, cols, c16, cbase, vals, p, q, part);
+  k_spmv_pq_k<S, NR, LPR, U, NW><<<grid, kTileThreads, 0, s>>>(T, st, row_ptr, cols, c16, cbase, vals, p, q, part, F);
 }
 template <class S, int NR, int LPR, int U>
 void launch_spmv(cudaStream_t s, unsigned grid, const Tiles& T, const ChartState* st, const DevSystem& sys,
-                 const S* vals, const S* p, S* q, double* part) {
+                 const S* vals, const S* p, S* q, double* part, const ChartStep& F = ChartStep()) {
   if (sys.cols16 && sys.rowrel16)
-    launch_spmv_nw<S, NR, LPR, U, 2>(s, grid, T, st, sys.row_ptr, sys.cols, sys.cols16, sys.cbase, vals, p, q, part);
+    launch_spmv_nw<S, NR, LPR, U, 2>(s, grid, T, st, sys.row_ptr, sys.cols, sys.cols16, sys.cbase, vals, p, q, part, F);
   else if (sys.cols16)
-    launch_spmv_nw<S, NR, LPR, U, 1>(s, grid, T, st, sys.row_ptr, sys.cols, sys.cols16, sys.cbase, vals, p, q, part);
+    launch_spmv_nw<S, NR, LPR, U, 1>(s, grid, T, st, sys.row_ptr, sys.cols, sys.cols16, sys.cbase, vals, p, q, part, F);
   else
-    launch_spmv_nw<S, NR, LPR, U, 0>(s, grid, T, st, sys.row_ptr, sys.cols, sys.cols16, sys.cbase, vals, p, q, part);
+    launch_spmv_nw<S, NR, LPR, U, 0>(s, grid, T, st, sys.row_ptr, sys.cols, sys.cols16, sys.cbase, vals, p, q, part, F);
 }
 
 // Allows the bulk-copy kernels the dynamic shared memory they need (outside any capture).
@@ -446,10 +584,11 @@ __global__ void __launch_bounds__(kTileThreads) k_update(Tiles T, const ChartSta
                                                          const S* __restrict__ dinv, int use_jacobi,
                                                          S* __restrict__ x, S* __restrict__ r, S* __restrict__ z,
                                                          const S* __restrict__ p, const S* __restrict__ q,
-                                                         double* __restrict__ part) {
+                                                         double* __restrict__ part, ChartStep F = ChartStep()) {
   __shared__ S sh[2 * 32];
   int64_t t = blockIdx.x;
-  const ChartState& cs = st[T.chart[t]];
+  const int32_t ch = T.chart[t];
+  const ChartState& cs = st[ch];
   if (cs.state != kActive) return;
   const S alpha = std::is_same<S, float>::value ? (S)cs.alpha32 : (S)cs.alpha;
   S acc[2] = {S(0), S(0)};
@@ -468,11 +607,9 @@ __global__ void __launch_bounds__(kTileThreads) k_update(Tiles T, const ChartSta
     stv<S, NR>(r, i, rv);
     if (use_jacobi != 2) stv<S, NR>(z, i, zv);
   }
-  block_sum_t<2, S>(acc, sh);
-  if (threadIdx.x == 0) {
-    part[2 * t] = (double)acc[0];
-    part[2 * t + 1] = (double)acc[1];
-  }
+  block_sum_first<2, S>(acc, sh);
+  const double v[2] = {(double)acc[0], (double)acc[1]};
+  tile_end<2>(T, F, t, ch, v, part);
 }
 
 // p = z + beta p
@@ -556,7 +693,7 @@ __global__ void __launch_bounds__(kTileThreads) k_true_residual(Tiles T, const C
                                                                 const float* __restrict__ bdf, const float* __restrict__ dinv,
                                                                 int precond, const float* __restrict__ xdf,
                                                                 float* __restrict__ r, float* __restrict__ z,
-                                                                double* __restrict__ part) {
+                                                                double* __restrict__ part, ChartStep F) {
   constexpr int K = (8 + LPR - 1) / LPR;
   __shared__ float sh[2 * 32];
   const int64_t t = blockIdx.x;
@@ -659,26 +796,51 @@ __global__ void __launch_bounds__(kTileThreads) k_true_residual(Tiles T, const C
   if constexpr (NW == 1) run(ColsNarrow{c16, cbase[T.chart[t]]});
   else if constexpr (NW == 2) run(ColsRowRel{c16});
   else run(ColsWide{cols});
-  block_sum_t<2, float>(acc, sh);
+  block_sum_first<2, float>(acc, sh);
+  double v[2] = {0.0, 0.0};
   if (threadIdx.x == 0) {
     const double inv = 1.0 / ((double)rsc * (double)rsc);
-    part[2 * t] = (double)acc[0] * inv;
-    part[2 * t + 1] = (double)acc[1] * inv;
+    v[0] = (double)acc[0] * inv;
+    v[1] = (double)acc[1] * inv;
   }
+  tile_end<2>(T, F, t, T.chart[t], v, part);
 }
 
 // One launch of the true residual for the system's column stream kind.
 template <int NR, int LPR, int U, class MX>
 void launch_true_residual(cudaStream_t s, unsigned grid, const Tiles& T, const ChartState* st, const DevSystem& sys,
-                          const MX& mx, const float* dinv32, int precond, float* r, float* z, double* part) {
+                          const MX& mx, const float* dinv32, int precond, float* r, float* z, double* part,
+                          const ChartStep& F) {
 #define RUV_TR(NWV)                                                                                                   \
   k_true_residual<NR, LPR, U, NWV><<<grid, kTileThreads, 0, s>>>(T, st, sys.row_ptr, sys.cols, sys.cols16, sys.cbase, \
                                                                 sys.vals32, mx.vals_lo, mx.rsum, mx.bdf, dinv32,      \
-                                                                precond, mx.xdf, r, z, part)
+                                                                precond, mx.xdf, r, z, part, F)
   if (sys.cols16 && sys.rowrel16) RUV_TR(2);
   else if (sys.cols16) RUV_TR(1);
   else RUV_TR(0);
 #undef RUV_TR
+}
+
+template <class S, int NR>
+__global__ void __launch_bounds__(kTileThreads) k_dots_rz(Tiles T, const ChartState* __restrict__ st, const S* __restrict__ r,
+                                                          const S* __restrict__ z, const S* __restrict__ q,
+                                                          double* __restrict__ part, ChartStep F = ChartStep()) {
+  __shared__ S sh[2 * 32];
+  int64_t t = blockIdx.x;
+  const int32_t ch = T.chart[t];
+  if (st[ch].state != kActive) return;
+  S acc[2] = {S(0), S(0)};
+  for (int64_t i = T.tab[2 * t] + threadIdx.x; i < T.tab[2 * t + 1]; i += blockDim.x) {
+    const V<S, NR> rv = ldv<S, NR>(r, i), zv = ldv<S, NR>(z, i), qv = ldv<S, NR>(q, i);
+#pragma unroll
+    for (int k = 0; k < NR; ++k) {
+      acc[0] += rv.c[k] * zv.c[k];
+      acc[1] += zv.c[k] * qv.c[k];
+    }
+  }
+  block_sum_first<2, S>(acc, sh);
+  const double v[2] = {(double)acc[0], (double)acc[1]};
+  tile_end<2>(T, F, t, ch, v, part);
 }
 
 // ---------------------------------------------------------------- chart kernels
@@ -724,126 +886,15 @@ __global__ void __launch_bounds__(kChartThreads) k_chart_init(Tiles T, ChartStat
   st[c] = s;
 }
 
-__global__ void __launch_bounds__(kChartThreads) k_chart_alpha(Tiles T, ChartState* __restrict__ st, const double* __restrict__ part,
-                                                               int* __restrict__ n_active) {
-  __shared__ double sh[32];
-  int64_t c = blockIdx.x;
-  if (st[c].state != kActive) return;
-  double v[1];
-  chart_reduce<1>(T, c, part, 1, v, sh);
-  if (threadIdx.x != 0) return;
-  ChartState& s = st[c];
-  double pap = v[0];
-  if (fabs(pap) <= 1e-300 || !isfinite(pap)) {  // solver.rs:505-508
-    s.status = RUV_ERR_BREAKDOWN;
-    s.state = kDone;
-    atomicSub(n_active, 1);
-    return;
-  }
-  s.alpha = s.rz / pap;
-  s.alpha32 = (float)s.alpha;
-}
-
-// FP64 path: convergence on the recurrence residual (solver.rs:518-522), then beta.
-__global__ void __launch_bounds__(kChartThreads) k_chart_beta(Tiles T, ChartState* __restrict__ st, const double* __restrict__ part,
-                                                              int precond_none, int64_t max_iter, int* __restrict__ n_active) {
-  __shared__ double sh[2 * 32];
-  int64_t c = blockIdx.x;
-  if (st[c].state != kActive) return;
-  double v[2];
-  chart_reduce<2>(T, c, part, 2, v, sh);
-  if (threadIdx.x != 0) return;
-  ChartState& s = st[c];
-  s.iters += 1;
-  s.rr = v[0];
-  if (sqrt(v[0]) <= s.tol_abs) {
-    s.status = RUV_OK;
-    s.state = kDone;
-    atomicSub(n_active, 1);
-    return;
-  }
-  if (s.iters >= max_iter) {
-    s.status = RUV_ERR_NOT_CONVERGED;
-    s.state = kDone;
-    atomicSub(n_active, 1);
-    return;
-  }
-  double rznew = precond_none ? v[0] : v[1];
-  s.beta = rznew / s.rz;
-  s.beta32 = (float)s.beta;
-  s.rz = rznew;
-}
-
-// Mixed path: the FP32 residual only schedules true-residual refreshes.
-__global__ void __launch_bounds__(kChartThreads) k_chart_beta_mixed(Tiles T, ChartState* __restrict__ st,
-                                                                    const double* __restrict__ part, int precond_none,
-                                                                    int64_t max_iter, int* __restrict__ n_active,
-                                                                    int separate_precond, double delta) {
-  __shared__ double sh[2 * 32];
-  int64_t c = blockIdx.x;
-  if (st[c].state != kActive) return;
-  double v[2];
-  chart_reduce<2>(T, c, part, 2, v, sh);
-  if (threadIdx.x != 0) return;
-  ChartState& s = st[c];
-  s.iters += 1;
-  double rn = sqrt(v[0]);
-  double rznew = precond_none ? v[0] : v[1];
-  if (rn <= delta * s.r_ref || rn <= s.tol_abs || !isfinite(rn) || s.iters >= max_iter) {
-    s.refresh = 1;  // beta is formed after the refresh, from the true residual
-  } else {
-    s.refresh = 0;
-    if (!separate_precond) {  // (a separate preconditioner forms beta after its apply)
-      s.beta = rznew / s.rz;
-      s.beta32 = (float)s.beta;
-      s.rz = rznew;
-    }
-  }
-  (void)n_active;
-}
-
-__global__ void __launch_bounds__(kChartThreads) k_chart_after_refresh(Tiles T, ChartState* __restrict__ st,
-                                                                       const double* __restrict__ part, int precond_none,
-                                                                       int64_t max_iter, int* __restrict__ n_active,
-                                                                       int separate_precond) {
-  __shared__ double sh[2 * 32];
-  int64_t c = blockIdx.x;
-  if (st[c].state != kActive || !st[c].refresh) return;
-  double v[2];
-  chart_reduce<2>(T, c, part, 2, v, sh);
-  if (threadIdx.x != 0) return;
-  ChartState& s = st[c];
-  s.refinements += 1;
-  s.rr = v[0];
-  double rn = sqrt(v[0]);
-  if (rn <= s.tol_abs) {
-    s.status = RUV_OK;
-    s.state = kDone;
-    atomicSub(n_active, 1);
-    return;
-  }
-  if (!isfinite(rn)) {
-    s.status = RUV_ERR_BREAKDOWN;
-    s.state = kDone;
-    atomicSub(n_active, 1);
-    return;
-  }
-  if (s.iters >= max_iter) {
-    s.status = RUV_ERR_NOT_CONVERGED;
-    s.state = kDone;
-    atomicSub(n_active, 1);
-    return;
-  }
-  s.r_ref = rn;
-  if (separate_precond) {
-    s.refresh = 2;  // refreshed: the beta kernel uses the plain Fletcher-Reeves ratio
-    return;
-  }
-  double rznew = precond_none ? v[0] : v[1];
-  s.beta = rznew / s.rz;
-  s.beta32 = (float)s.beta;
-  s.rz = rznew;
-  s.refresh = 0;
+// A chart step as a kernel of its own, one CTA per chart.
+template <int NV>
+__global__ void __launch_bounds__(kChartThreads) k_chart_step(Tiles T, ChartStep F, const double* __restrict__ part) {
+  __shared__ double sh[NV * 32];
+  const int64_t c = blockIdx.x;
+  if (F.st[c].state != kActive || (F.kind == kStepAfterRefresh && !F.st[c].refresh)) return;
+  double v[NV];
+  chart_reduce<NV>(T, c, part, NV, v, sh);
+  if (threadIdx.x == 0) chart_step(F, c, v[0], NV > 1 ? v[NV - 1] : 0.0);
 }
 
 // ---------------------------------------------------------------- separate preconditioner
@@ -854,29 +905,6 @@ __global__ void k_mark_done(const ChartState* __restrict__ st, int64_t n, int32_
 }
 
 template <class S, int NR>
-__global__ void __launch_bounds__(kTileThreads) k_dots_rz(Tiles T, const ChartState* __restrict__ st, const S* __restrict__ r,
-                                                          const S* __restrict__ z, const S* __restrict__ q,
-                                                          double* __restrict__ part) {
-  __shared__ S sh[2 * 32];
-  int64_t t = blockIdx.x;
-  if (st[T.chart[t]].state != kActive) return;
-  S acc[2] = {S(0), S(0)};
-  for (int64_t i = T.tab[2 * t] + threadIdx.x; i < T.tab[2 * t + 1]; i += blockDim.x) {
-    const V<S, NR> rv = ldv<S, NR>(r, i), zv = ldv<S, NR>(z, i), qv = ldv<S, NR>(q, i);
-#pragma unroll
-    for (int k = 0; k < NR; ++k) {
-      acc[0] += rv.c[k] * zv.c[k];
-      acc[1] += zv.c[k] * qv.c[k];
-    }
-  }
-  block_sum_t<2, S>(acc, sh);
-  if (threadIdx.x == 0) {
-    part[2 * t] = (double)acc[0];
-    part[2 * t + 1] = (double)acc[1];
-  }
-}
-
-template <class S, int NR>
 __global__ void __launch_bounds__(kTileThreads) k_copy_dir(Tiles T, const ChartState* __restrict__ st, const S* __restrict__ z,
                                                            S* __restrict__ p) {
   int64_t t = blockIdx.x;
@@ -884,71 +912,11 @@ __global__ void __launch_bounds__(kTileThreads) k_copy_dir(Tiles T, const ChartS
   for (int64_t i = T.tab[2 * t] + threadIdx.x; i < T.tab[2 * t + 1]; i += blockDim.x) stv<S, NR>(p, i, ldv<S, NR>(z, i));
 }
 
-// FP64 outer loop with a separate preconditioner: convergence on the recurrence residual
-// (solver.rs:518-522); beta comes after the apply.
-__global__ void __launch_bounds__(kChartThreads) k_chart_check64(Tiles T, ChartState* __restrict__ st,
-                                                                 const double* __restrict__ part, int64_t max_iter,
-                                                                 int* __restrict__ n_active) {
-  __shared__ double sh[2 * 32];
-  int64_t c = blockIdx.x;
-  if (st[c].state != kActive) return;
-  double v[2];
-  chart_reduce<2>(T, c, part, 2, v, sh);
-  if (threadIdx.x != 0) return;
-  ChartState& s = st[c];
-  s.iters += 1;
-  s.rr = v[0];
-  if (sqrt(v[0]) <= s.tol_abs) {
-    s.status = RUV_OK;
-    s.state = kDone;
-    atomicSub(n_active, 1);
-  } else if (!isfinite(v[0])) {
-    s.status = RUV_ERR_BREAKDOWN;
-    s.state = kDone;
-    atomicSub(n_active, 1);
-  } else if (s.iters >= max_iter) {
-    s.status = RUV_ERR_NOT_CONVERGED;
-    s.state = kDone;
-    atomicSub(n_active, 1);
-  }
-}
-
 // FP64 <-> FP32 copies of the preconditioner's input / output (FP64 outer loop).
 template <class A, class Bt>
 __global__ void k_convert(int64_t n, const A* __restrict__ in, Bt* __restrict__ out) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = (Bt)in[i];
-}
-
-// After the first apply: rz = r.z.
-__global__ void __launch_bounds__(kChartThreads) k_chart_rz0(Tiles T, ChartState* __restrict__ st, const double* __restrict__ part) {
-  __shared__ double sh[2 * 32];
-  int64_t c = blockIdx.x;
-  if (st[c].state != kActive) return;
-  double v[2];
-  chart_reduce<2>(T, c, part, 2, v, sh);
-  if (threadIdx.x == 0) st[c].rz = v[0];
-}
-
-// beta after a separate apply: flexible (Polak-Ribiere, as the reference's FCG for AMG,
-// solver.rs:474-481, :526-539) using r_new - r_old = -alpha q, or Fletcher-Reeves right
-// after a true-residual refresh (r jumped).
-__global__ void __launch_bounds__(kChartThreads) k_chart_beta_pc(Tiles T, ChartState* __restrict__ st,
-                                                                 const double* __restrict__ part, int flexible) {
-  __shared__ double sh[2 * 32];
-  int64_t c = blockIdx.x;
-  if (st[c].state != kActive) return;
-  double v[2];
-  chart_reduce<2>(T, c, part, 2, v, sh);
-  if (threadIdx.x != 0) return;
-  ChartState& s = st[c];
-  const double rznew = v[0];
-  double beta = (flexible && s.refresh != 2) ? (-s.alpha * v[1]) / s.rz : rznew / s.rz;
-  if (!isfinite(beta)) beta = 0.0;
-  s.beta = beta;
-  s.beta32 = (float)beta;
-  s.rz = rznew;
-  s.refresh = 0;
 }
 
 // ---------------------------------------------------------------- host driver
@@ -987,6 +955,18 @@ MixedExtras mixed_extras(Ctx& ctx, DevSystem& sys, int nr) {
   }
   return m;
 }
+
+// The chart steps' arrival counters, zero (a step leaves them so; a failed solve may not have).
+int32_t* arrived_counters(Ctx& ctx, int64_t n_charts) {
+  int32_t* d = ctx.ws.get<int32_t>("pcg.arrived", n_charts);
+  RUV_CUDA(cudaMemsetAsync(d, 0, sizeof(int32_t) * std::max<int64_t>(n_charts, 1), ctx.stream));
+  return d;
+}
+
+// Whether the tile kernels take the chart steps: up to eight tiles an SM.  With more, the fence and the
+// atomic that end every tile cost the kernels' throughput more than a kernel between them costs (4096
+// disks, 14,900 tiles: 110 against 106 ms; a 1024^2 field's 1,021 tiles 35.7 against 35.1).
+inline bool steps_in_tiles(const Ctx& ctx, int64_t n_tiles) { return n_tiles <= 8 * (int64_t)ctx.sm_count; }
 
 template <class S, int NR, int LPR, int U>
 void run_pcg(Ctx& ctx, DevSystem& sys, double* x64, const SolveOpts& o, Tiles T, ChartState* st, int* n_active,
@@ -1039,24 +1019,42 @@ void run_pcg(Ctx& ctx, DevSystem& sys, double* x64, const SolveOpts& o, Tiles T,
     RUV_CUDA(cudaStreamSynchronize(s));
   }
   if (*h_active > 0) {
+    ChartStep base;
+    base.precond_none = none;
+    base.max_iter = o.max_iter;
+    base.delta = refresh_delta();
+    base.st = st;
+    base.n_active = n_active;
+    base.arrived = arrived_counters(ctx, NC);
+    const bool in_tiles = steps_in_tiles(ctx, NTL);
+    auto step = [&](int kind) {
+      ChartStep f = base;
+      f.kind = in_tiles ? kind : kStepNone;
+      return f;
+    };
+    auto chart = [&](auto nv, int kind) {  // the step's own kernel where the tiles do not take it
+      if (in_tiles) return;
+      ChartStep f = base;
+      f.kind = kind;
+      k_chart_step<decltype(nv)::value><<<(unsigned)NC, kChartThreads, 0, s>>>(T, f, part);
+    };
+    constexpr std::integral_constant<int, 1> one{};
+    constexpr std::integral_constant<int, 2> two{};
     // capture kCheckEvery iterations as one graph, replay it
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     RUV_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     for (int rep = 0; rep < kCheckEvery; ++rep) {
-      launch_spmv<S, NR, LPR, U>(s, (unsigned)NTL, T, st, sys, vals, p, q, part);
-      k_chart_alpha<<<(unsigned)NC, kChartThreads, 0, s>>>(T, st, part, n_active);
+      launch_spmv<S, NR, LPR, U>(s, (unsigned)NTL, T, st, sys, vals, p, q, part, step(kStepAlpha));
+      chart(one, kStepAlpha);
       k_update<S, NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, dinv, jac, mixed ? xs : reinterpret_cast<S*>(x64), r,
-                                                             z, p, q, part);
-      if (!mixed) {
-        k_chart_beta<<<(unsigned)NC, kChartThreads, 0, s>>>(T, st, part, none, o.max_iter, n_active);
-      } else {
-        k_chart_beta_mixed<<<(unsigned)NC, kChartThreads, 0, s>>>(T, st, part, none, o.max_iter, n_active, 0,
-                                                                  refresh_delta());
+                                                             z, p, q, part, step(mixed ? kStepBetaMixed : kStepBeta));
+      chart(two, mixed ? kStepBetaMixed : kStepBeta);
+      if (mixed) {
         k_fold<NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, 0, mx.xdf, reinterpret_cast<float*>(xs), x64);
         launch_true_residual<NR, LPR, U>(s, (unsigned)NTL, T, st, sys, mx, dinv32, jac, reinterpret_cast<float*>(r),
-                                         reinterpret_cast<float*>(z), part);
-        k_chart_after_refresh<<<(unsigned)NC, kChartThreads, 0, s>>>(T, st, part, none, o.max_iter, n_active, 0);
+                                         reinterpret_cast<float*>(z), part, step(kStepAfterRefresh));
+        chart(two, kStepAfterRefresh);
       }
       k_direction<S, NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, z, p);
     }
@@ -1071,7 +1069,7 @@ void run_pcg(Ctx& ctx, DevSystem& sys, double* x64, const SolveOpts& o, Tiles T,
     try {
       while (launched < o.max_iter + kCheckEvery) {
         RUV_CUDA(cudaGraphLaunch(exec, s));
-        count_launches((int64_t)kCheckEvery * (mixed ? 8 : 5));
+        count_launches((int64_t)kCheckEvery * ((mixed ? 5 : 3) + (in_tiles ? 0 : mixed ? 3 : 2)));
         launched += kCheckEvery;
         RUV_CUDA(cudaMemcpyAsync(h_active, n_active, sizeof(int), cudaMemcpyDeviceToHost, s));
         if (T.err) RUV_CUDA(cudaMemcpyAsync(h_active + 2, T.err, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -1175,10 +1173,34 @@ void run_pcg_sep(Ctx& ctx, DevSystem& sys, double* x64, const SolveOpts& o, Tile
     to32();
     count_launches(1 + conv + P.apply(ctx, done));
     to64();
-    k_dots_rz<S, NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, r, z, q, part2);
-    k_chart_rz0<<<(unsigned)NC, kChartThreads, 0, s>>>(T, st, part2);
+    ChartStep base;
+    base.precond_none = base.separate = 1;
+    base.flexible = flex;
+    base.max_iter = o.max_iter;
+    base.delta = refresh_delta();
+    base.st = st;
+    base.n_active = n_active;
+    base.done = done;
+    base.arrived = arrived_counters(ctx, NC);
+    const bool in_tiles = steps_in_tiles(ctx, NTL);
+    auto step = [&](int kind) {
+      ChartStep f = base;
+      f.kind = in_tiles ? kind : kStepNone;
+      return f;
+    };
+    auto chart = [&](auto nv, int kind, const double* sums) -> int {  // (its own kernel, where the tiles do not)
+      if (in_tiles) return 0;
+      ChartStep f = base;
+      f.kind = kind;
+      k_chart_step<decltype(nv)::value><<<(unsigned)NC, kChartThreads, 0, s>>>(T, f, sums);
+      return 1;
+    };
+    constexpr std::integral_constant<int, 1> one{};
+    constexpr std::integral_constant<int, 2> two{};
+    k_dots_rz<S, NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, r, z, q, part2, step(kStepRz0));
+    count_launches(chart(two, kStepRz0, part2));
     k_copy_dir<S, NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, z, p);
-    count_launches(3);
+    count_launches(2);
     RUV_LAUNCH_CHECK();
     constexpr int kRep = 8;
     cudaGraph_t graph = nullptr;
@@ -1187,30 +1209,25 @@ void run_pcg_sep(Ctx& ctx, DevSystem& sys, double* x64, const SolveOpts& o, Tile
     RUV_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     for (int rep = 0; rep < kRep; ++rep) {
       int l = 0;
-      launch_spmv<S, NR, LPR, U>(s, (unsigned)NTL, T, st, sys, vals, p, q, part);
-      k_chart_alpha<<<(unsigned)NC, kChartThreads, 0, s>>>(T, st, part, n_active);
-      k_update<S, NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, dinv, 2, xiter, r, z, p, q, part);
+      launch_spmv<S, NR, LPR, U>(s, (unsigned)NTL, T, st, sys, vals, p, q, part, step(kStepAlpha));
+      l += chart(one, kStepAlpha, part);
+      k_update<S, NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, dinv, 2, xiter, r, z, p, q, part,
+                                                             step(mixed ? kStepBetaMixed : kStepCheck64));
+      l += chart(two, mixed ? kStepBetaMixed : kStepCheck64, part);
       if (mixed) {
-        k_chart_beta_mixed<<<(unsigned)NC, kChartThreads, 0, s>>>(T, st, part, 1, o.max_iter, n_active, 1,
-                                                                  refresh_delta());
         k_fold<NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, 0, mx.xdf, reinterpret_cast<float*>(xs), x64);
         launch_true_residual<NR, LPR, U>(s, (unsigned)NTL, T, st, sys, mx, dinv32, 2, reinterpret_cast<float*>(r),
-                                         reinterpret_cast<float*>(z), part);
-        k_chart_after_refresh<<<(unsigned)NC, kChartThreads, 0, s>>>(T, st, part, 1, o.max_iter, n_active, 1);
-        l += 4;
-      } else {
-        k_chart_check64<<<(unsigned)NC, kChartThreads, 0, s>>>(T, st, part, o.max_iter, n_active);
-        l += 1;
+                                         reinterpret_cast<float*>(z), part, step(kStepAfterRefresh));
+        l += 2 + chart(two, kStepAfterRefresh, part);
       }
-      k_mark_done<<<div_up(NC, 256), 256, 0, s>>>(st, NC, done);
       to32();
-      l += 4 + conv;
+      l += 2 + conv;
       l += P.apply(ctx, done);
       to64();
-      k_dots_rz<S, NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, r, z, q, part2);
-      k_chart_beta_pc<<<(unsigned)NC, kChartThreads, 0, s>>>(T, st, part2, flex);
+      k_dots_rz<S, NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, r, z, q, part2, step(kStepBetaPc));
+      l += chart(two, kStepBetaPc, part2);
       k_direction<S, NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, z, p);
-      l += 3;
+      l += 2;
       per_iter = l;
     }
     cudaError_t ce = cudaStreamEndCapture(s, &graph);
@@ -1279,15 +1296,22 @@ void dispatch_pcg(Shape sh, Ctx& ctx, DevSystem& sys, double* x64, const SolveOp
 
 TileTable make_tiles(const std::vector<int64_t>& chart_row, int64_t tile_rows);
 
-// Rows per tile of a solve: the context's, or in the mixed loop, where none was chosen and a system is
-// too small to give every SM four tiles of that size, down to 128.  (The FP64 loop keeps its tiles: its
-// block sums occupy the FP64 pipe, and 128-row tiles took a 89,401-row chart from 27 to 36 us an
-// iteration.)
+// Rows per tile of a solve: the context's where one was chosen.  Else, for a system too small to give
+// every SM four tiles of the default size: the mixed loop halves them, down to 128; the FP64 loop, which
+// the SMs' FP64 pipes bound, splits a large chart evenly -- a tile an SM, or as few more as keep them
+// at about the default -- since the SM with most rows is the one waited for (89,401 rows in 88 tiles
+// of 1024 left 64 SMs idle: 55 -> 49 ms; 160,000 in 157 gave five SMs twice the rows: 17.3 -> 14.9 ms)
+// and smaller tiles only add block sums (128 rows: 65 ms).
 int64_t solve_tile_rows(const Ctx& ctx, const DevSystem& sys, bool mixed) {
   int64_t tile = ctx.tile_rows;
-  if (mixed && !ctx.tile_set)
+  if (ctx.tile_set || sys.n_rows >= 4 * tile * ctx.sm_count) return tile;
+  if (mixed) {
     while (tile > 128 && sys.n_rows < 4 * tile * ctx.sm_count) tile /= 2;
-  return tile;
+    return tile;
+  }
+  const int64_t per_sm = std::max<int64_t>(1, (sys.n_rows + 1100 * ctx.sm_count - 1) / (1100 * ctx.sm_count));
+  const int64_t even = (sys.n_rows + per_sm * ctx.sm_count - 1) / (per_sm * ctx.sm_count);
+  return std::max<int64_t>(512, (even + 15) & ~(int64_t)15);
 }
 
 Tiles upload_tiles(Ctx& ctx, const DevSystem& sys, const std::string& tag, int64_t tile_rows) {
@@ -1333,10 +1357,13 @@ Tiles upload_tiles(Ctx& ctx, const DevSystem& sys, const std::string& tag, int64
 // The launch shape without the autotuner: for mesh Laplacians (at most 8 entries per row) two
 // lanes per row and two rows in flight, which the autotuner picked on every such operator
 // measured (4096 disks, 1024^2 and 2048^2 height fields); wider sub-warps for denser rows.
-Shape pick_shape(const Ctx& ctx, const DevSystem& sys) {
+Shape pick_shape(const Ctx& ctx, const DevSystem& sys, bool one_lane = false) {
   double avg = sys.n_rows > 0 ? (double)sys.nnz / (double)sys.n_rows : 1.0;
   int lpr = ctx.lanes_per_row > 0 ? ctx.lanes_per_row : (avg <= 8 ? 2 : avg <= 12 ? 8 : avg <= 24 ? 16 : 32);
   int u = ctx.unroll > 0 ? ctx.unroll : (lpr <= 4 ? 2 : lpr == 8 ? 4 : 1);
+  // FP64: one lane per row, whose sum needs no additions across lanes (a quarter of a two-lane row's FP64
+  // instructions): 49.0 -> 47.5 ms on an 89,401-row chart, 14.9 -> 14.3 ms on 160,000 rows
+  if (one_lane && ctx.lanes_per_row == 0 && lpr == 2) lpr = 1;
   return Shape{lpr, u};
 }
 
@@ -1594,9 +1621,9 @@ std::vector<ChartResult> pcg_solve(Ctx& ctx, DevSystem& sys, double* x, const So
   Tiles T = upload_tiles(ctx, sys, "pcg", o.teams ? solve_tile_rows(ctx, sys, o.precision == RUV_PREC_MIXED) : ctx.tile_rows);
   ChartState* st = ctx.ws.get<ChartState>("pcg.state", NC);
   int* n_active = ctx.ws.get<int>("pcg.nactive", 1);
-  const Shape sh = pick_shape(ctx, sys);
-  std::vector<ChartState> out;
   const bool mixed = o.precision == RUV_PREC_MIXED;
+  const Shape sh = pick_shape(ctx, sys, !mixed && o.teams);
+  std::vector<ChartState> out;
   ctx.timings[3] = 0.0;
   if (sep) {
     // preconditioner set-up, timed on the stream
@@ -1731,10 +1758,17 @@ template <int LPR, int U>
 void na_iterations(cudaStream_t s, NoAllocScratch* S, Tiles T, const int32_t* row_ptr, const int32_t* cols,
                    const double* vals, double* x, int jac, int none, int64_t max_iter) {
   k_spmv_pq_k<double, 1, LPR, U, false><<<(unsigned)T.n, kTileThreads, 0, s>>>(T, &S->st, row_ptr, cols, nullptr, nullptr,
-                                                                              vals, S->p, S->q, S->part);
-  k_chart_alpha<<<1, kChartThreads, 0, s>>>(T, &S->st, S->part, &S->n_active);
+                                                                              vals, S->p, S->q, S->part, ChartStep());
+  ChartStep f;
+  f.precond_none = none;
+  f.max_iter = max_iter;
+  f.st = &S->st;
+  f.n_active = &S->n_active;
+  f.kind = kStepAlpha;
+  k_chart_step<1><<<1, kChartThreads, 0, s>>>(T, f, S->part);
   k_update<double, 1><<<(unsigned)T.n, kTileThreads, 0, s>>>(T, &S->st, S->dinv, jac, x, S->r, S->z, S->p, S->q, S->part);
-  k_chart_beta<<<1, kChartThreads, 0, s>>>(T, &S->st, S->part, none, max_iter, &S->n_active);
+  f.kind = kStepBeta;
+  k_chart_step<2><<<1, kChartThreads, 0, s>>>(T, f, S->part);
   k_direction<double, 1><<<(unsigned)T.n, kTileThreads, 0, s>>>(T, &S->st, S->z, S->p);
 }
 
