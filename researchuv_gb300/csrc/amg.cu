@@ -41,6 +41,13 @@ constexpr float kOmega = 2.0f / 3.0f;
 // save about 2.3 ms of set-up on the 4096-disk step and 11 ms on the 2048^2 field's step
 // (fewer iterations there too: 130 against 138)
 constexpr int kPairRounds = 3;
+// From this many rows on, a level's matching passes take two rounds and a third level gets a smoothed
+// prolongator: set-up and cycles stream HBM there, and what they save is more than the iterations they
+// cost (4096 disks: set-up 29.3 -> 24.6 ms, iterations 26 / 15.4 -> 27 / 17.9, solve 103.2 -> 99.1 ms; 1024^2
+// field 92 -> 87 iterations, 30.7 -> 28.4 ms).  Below, steps cost their latency whatever their rows, and
+// iterations count: a 300^2 chart 52 -> 62 iterations, 11.9 -> 13.0 ms.
+constexpr int64_t kLargeRows = 500000;
+constexpr int kLargeRounds = 2, kLargeSaLevels = 3;
 // distinct keys per accumulated strength row: group strengths beyond it (only on dense coarse
 // levels of the smoothed hierarchy) are left out of the matching, deterministically
 constexpr int kAccCap = 48;
@@ -1239,7 +1246,7 @@ __global__ void __launch_bounds__(kAmgThreads) k_smooth_down(LvlTiles T, const i
                                                              const int32_t* __restrict__ cbase,
                                                              const float* __restrict__ vals, const float* __restrict__ dinv,
                                                              const float* __restrict__ b, float* __restrict__ x,
-                                                             float* __restrict__ t) {
+                                                             float* __restrict__ t, float omega) {
   const int64_t tl = blockIdx.x;
   const int32_t ch = T.chart[tl];
   if (done[ch]) return;
@@ -1248,7 +1255,7 @@ __global__ void __launch_bounds__(kAmgThreads) k_smooth_down(LvlTiles T, const i
       T.tab[2 * tl], T.tab[2 * tl + 1], nullptr, rp, colf, [&](int64_t e) { return vals[e]; },
       [&](int32_t j) {
         F<NR> v = ldf<NR>(b, j);
-        const float wd = kOmega * dinv[j];
+        const float wd = omega * dinv[j];
 #pragma unroll
         for (int c = 0; c < NR; ++c) v.c[c] *= wd;
         return v;
@@ -1256,7 +1263,7 @@ __global__ void __launch_bounds__(kAmgThreads) k_smooth_down(LvlTiles T, const i
       [&](int64_t i, const F<NR>& s) {
         const F<NR> bi = ldf<NR>(b, i);
         F<NR> xi, ti;
-        const float wd = kOmega * dinv[i];
+        const float wd = omega * dinv[i];
 #pragma unroll
         for (int c = 0; c < NR; ++c) {
           xi.c[c] = wd * bi.c[c];
@@ -1297,7 +1304,7 @@ __global__ void __launch_bounds__(kAmgThreads) k_smooth_down_st(LvlTiles T, cons
                                                                 const float* __restrict__ vals,
                                                                 const float* __restrict__ dinv,
                                                                 const float* __restrict__ b, float* __restrict__ x,
-                                                                float* __restrict__ t, int64_t limit, int* err) {
+                                                                float* __restrict__ t, int64_t limit, int* err, float omega) {
   extern __shared__ __align__(16) unsigned char stage[];
   const int64_t tl = blockIdx.x;
   const int32_t ch = T.chart[tl];
@@ -1313,7 +1320,7 @@ __global__ void __launch_bounds__(kAmgThreads) k_smooth_down_st(LvlTiles T, cons
       [&](int64_t e) { return op.w(e); },
       [&](int32_t j) {
         F<NR> v = ldf<NR>(b, j);
-        const float wd = kOmega * dinv[j];
+        const float wd = omega * dinv[j];
 #pragma unroll
         for (int c = 0; c < NR; ++c) v.c[c] *= wd;
         return v;
@@ -1321,7 +1328,7 @@ __global__ void __launch_bounds__(kAmgThreads) k_smooth_down_st(LvlTiles T, cons
       [&](int64_t i, const F<NR>& sv) {
         const F<NR> bi = ldf<NR>(b, i);
         F<NR> xi, ti;
-        const float wd = kOmega * dinv[i];
+        const float wd = omega * dinv[i];
 #pragma unroll
         for (int c = 0; c < NR; ++c) {
           xi.c[c] = wd * bi.c[c];
@@ -1341,7 +1348,7 @@ __global__ void __launch_bounds__(kAmgThreads) k_smooth_up_st(LvlTiles T, const 
                                                               const float* __restrict__ vals,
                                                               const float* __restrict__ dinv,
                                                               const float* __restrict__ b, const float* __restrict__ y,
-                                                              float* __restrict__ x, int64_t limit, int* err) {
+                                                              float* __restrict__ x, int64_t limit, int* err, float omega) {
   extern __shared__ __align__(16) unsigned char stage[];
   const int64_t tl = blockIdx.x;
   const int32_t ch = T.chart[tl];
@@ -1358,7 +1365,7 @@ __global__ void __launch_bounds__(kAmgThreads) k_smooth_up_st(LvlTiles T, const 
       [&](int64_t i, const F<NR>& sv) {
         const F<NR> bi = ldf<NR>(b, i), yi = ldf<NR>(y, i);
         F<NR> xi;
-        const float wd = kOmega * dinv[i];
+        const float wd = omega * dinv[i];
 #pragma unroll
         for (int c = 0; c < NR; ++c) xi.c[c] = yi.c[c] + wd * (bi.c[c] - sv.c[c]);
         stf<NR>(x, i, xi);
@@ -1510,7 +1517,7 @@ __global__ void __launch_bounds__(kAmgThreads) k_smooth_up(LvlTiles T, const int
                                                            const int32_t* __restrict__ cbase,
                                                            const float* __restrict__ vals, const float* __restrict__ dinv,
                                                            const float* __restrict__ b, const float* __restrict__ y,
-                                                           float* __restrict__ x) {
+                                                           float* __restrict__ x, float omega) {
   const int64_t tl = blockIdx.x;
   const int32_t ch = T.chart[tl];
   if (done[ch]) return;
@@ -1521,7 +1528,7 @@ __global__ void __launch_bounds__(kAmgThreads) k_smooth_up(LvlTiles T, const int
       [&](int64_t i, const F<NR>& s) {
         const F<NR> bi = ldf<NR>(b, i), yi = ldf<NR>(y, i);
         F<NR> xi;
-        const float wd = kOmega * dinv[i];
+        const float wd = omega * dinv[i];
 #pragma unroll
         for (int c = 0; c < NR; ++c) xi.c[c] = yi.c[c] + wd * (bi.c[c] - s.c[c]);
         stf<NR>(x, i, xi);
@@ -1544,13 +1551,13 @@ __global__ void __launch_bounds__(kAmgThreads) k_smooth_up_t(LvlTiles T, const i
                                                              const float* __restrict__ vals, const float* __restrict__ dinv,
                                                              const float* __restrict__ b, const int32_t* __restrict__ agg,
                                                              const float* __restrict__ xc, float alpha_c,
-                                                             float* __restrict__ x) {
+                                                             float* __restrict__ x, float omega) {
   const int64_t tl = blockIdx.x;
   const int32_t ch = T.chart[tl];
   if (done[ch]) return;
   auto yval = [&](int64_t j) {
     F<NR> v = ldf<NR>(b, j);
-    const float wd = kOmega * dinv[j];
+    const float wd = omega * dinv[j];
     const F<NR> c = ldf<NR>(xc, agg[j]);
 #pragma unroll
     for (int k = 0; k < NR; ++k) v.c[k] = wd * v.c[k] + alpha_c * c.c[k];
@@ -1563,7 +1570,7 @@ __global__ void __launch_bounds__(kAmgThreads) k_smooth_up_t(LvlTiles T, const i
       [&](int64_t i, const F<NR>& s) {
         const F<NR> bi = ldf<NR>(b, i), yi = yval(i);
         F<NR> xi;
-        const float wd = kOmega * dinv[i];
+        const float wd = omega * dinv[i];
 #pragma unroll
         for (int c = 0; c < NR; ++c) xi.c[c] = yi.c[c] + wd * (bi.c[c] - s.c[c]);
         stf<NR>(x, i, xi);
@@ -1678,6 +1685,7 @@ struct AmgHierarchy {
   std::vector<int32_t> h_final;
   int64_t total_rows = 0, total_nnz = 0;
   float alpha_c = 1.0f;
+  float omega = kOmega;  // the smoothers' Jacobi weight
   int k_levels = 0;  // top levels applied in the K-form (two coarse corrections with steplengths)
   int* err = nullptr;  // a staged tile's bounded wait ran out
   int64_t spin_limit = 0;
@@ -1849,7 +1857,7 @@ void stage_setup(Ctx& ctx, AmgHierarchy* H) {
   L.stage_smem = bytes;
 }
 
-AmgHierarchy* amg_setup(Ctx& ctx, const DevSystem& sys, bool smooth, std::string& info) {
+AmgHierarchy* amg_setup(Ctx& ctx, const DevSystem& sys, bool smooth, std::string& info, bool first_form) {
   cudaStream_t s = ctx.stream;
   const int B = kAmgThreads;
   const int64_t NC = sys.n_charts;
@@ -1859,7 +1867,8 @@ AmgHierarchy* amg_setup(Ctx& ctx, const DevSystem& sys, bool smooth, std::string
   H->n_charts = NC;
   // smoothed prolongators on the first sa_levels levels, tentative below (the coarse levels of a
   // smoothed hierarchy are the densest: their products and cycles cost the most)
-  H->sa_levels = smooth ? kSaLevels : 0;
+  const bool by_size = !first_form;
+  H->sa_levels = !smooth ? 0 : by_size && sys.n_rows >= kLargeRows ? kLargeSaLevels : kSaLevels;
   if (const char* e = std::getenv("RUV_AMG_SA_LEVELS")) H->sa_levels = smooth ? std::max(0, std::atoi(e)) : 0;
   H->alpha_c = 1.5f;  // over-correct the piecewise-constant coarse space of tentative levels
   if (const char* e = std::getenv("RUV_AMG_ALPHA")) H->alpha_c = (float)std::atof(e);
@@ -1868,8 +1877,7 @@ AmgHierarchy* amg_setup(Ctx& ctx, const DevSystem& sys, bool smooth, std::string
   if (const char* e = std::getenv("RUV_AMG_STRONG")) strong = (float)std::atof(e);
   int pmax = kPMaxRow;
   if (const char* e = std::getenv("RUV_AMG_PMAX")) pmax = std::max(1, std::min(kAccCap, std::atoi(e)));
-  int rounds = kPairRounds;  // proposal rounds of each matching pass
-  if (const char* e = std::getenv("RUV_AMG_ROUNDS")) rounds = std::max(1, std::atoi(e));
+  const char* rounds_env = std::getenv("RUV_AMG_ROUNDS");  // proposal rounds of each matching pass
   // group matching over a group graph built once per level (RUV_AMG_GROUP_GRAPH=0: strengths
   // accumulated again in every round; the same aggregates)
   const char* gg_env = std::getenv("RUV_AMG_GROUP_GRAPH");
@@ -1946,6 +1954,8 @@ AmgHierarchy* amg_setup(Ctx& ctx, const DevSystem& sys, bool smooth, std::string
     RUV_CUDA(cudaStreamSynchronize(s));  // `cont` is reused by the next level
     if (n_cont == 0) break;
     // ---- aggregation: pairs of rows, then pairs of pairs
+    const int rounds = rounds_env ? std::max(1, std::atoi(rounds_env))
+                       : by_size && L.n >= kLargeRows ? kLargeRounds : kPairRounds;
     int32_t* mate = ctx.ws.get<int32_t>(tag + ".mate", L.n);
     int32_t* prop = ctx.ws.get<int32_t>(tag + ".prop", L.n);
     RUV_CUDA(cudaMemsetAsync(mate, 0xff, sizeof(int32_t) * L.n, s));
@@ -2265,7 +2275,7 @@ void amg_export_level(Ctx& ctx, const DevSystem& sys, bool smooth, int level, Am
     void operator()(AmgHierarchy* h) const { amg_free(h); }
   };
   std::string info;
-  std::unique_ptr<AmgHierarchy, Free> H(amg_setup(ctx, sys, smooth, info));
+  std::unique_ptr<AmgHierarchy, Free> H(amg_setup(ctx, sys, smooth, info, false));
   const int K = (int)H->lv.size();
   out = AmgLevelHost();
   out.n_levels = K;
@@ -2407,10 +2417,10 @@ int vtail(Ctx& ctx, AmgHierarchy* H, const int32_t* done, int k0) {
 #define CALL(X, UU, KK)                                                                                                \
   if (L.stage_smem)                                                                                                    \
     k_smooth_down_st<NR, X, UU, KK, NW><<<(unsigned)L.cont.n, B, L.stage_smem, s>>>(                                   \
-        L.cont, done, L.rp, L.cols, L.c16, L.cbase, L.vals, L.dinv, L.b, xpre, L.t, H->spin_limit, H->err);            \
+        L.cont, done, L.rp, L.cols, L.c16, L.cbase, L.vals, L.dinv, L.b, xpre, L.t, H->spin_limit, H->err, H->omega);            \
   else                                                                                                                 \
     k_smooth_down<NR, X, UU, KK, NW><<<(unsigned)L.cont.n, B, 0, s>>>(L.cont, done, L.rp, L.cols, L.c16, L.cbase, L.vals, \
-                                                                      L.dinv, L.b, xpre, L.t)
+                                                                      L.dinv, L.b, xpre, L.t, H->omega)
     if (L.c16 && L.rowrel) {
       constexpr int NW = 2;
       RUV_SMOOTH_SWITCH(la, CALL)
@@ -2441,7 +2451,7 @@ int vtail(Ctx& ctx, AmgHierarchy* H, const int32_t* done, int k0) {
     if (!L.smoothed) {
 #define CALL(X, UU, KK)                                                                                                \
   k_smooth_up_t<NR, X, UU, KK, NW><<<(unsigned)L.cont.n, B, 0, s>>>(L.cont, done, L.rp, L.cols, L.c16, L.cbase, L.vals, \
-                                                                    L.dinv, L.b, L.agg, C.x, H->alpha_c, L.x)
+                                                                    L.dinv, L.b, L.agg, C.x, H->alpha_c, L.x, H->omega)
       if (L.c16 && L.rowrel) {
         constexpr int NW = 2;
         RUV_SMOOTH_SWITCH(la, CALL)
@@ -2464,10 +2474,10 @@ int vtail(Ctx& ctx, AmgHierarchy* H, const int32_t* done, int k0) {
 #define CALL(X, UU, KK)                                                                                              \
   if (L.stage_smem)                                                                                                  \
     k_smooth_up_st<NR, X, UU, KK, NW><<<(unsigned)L.cont.n, B, L.stage_smem, s>>>(                                   \
-        L.cont, done, L.rp, L.cols, L.c16, L.cbase, L.vals, L.dinv, L.b, L.y, L.x, H->spin_limit, H->err);           \
+        L.cont, done, L.rp, L.cols, L.c16, L.cbase, L.vals, L.dinv, L.b, L.y, L.x, H->spin_limit, H->err, H->omega);           \
   else                                                                                                               \
     k_smooth_up<NR, X, UU, KK, NW><<<(unsigned)L.cont.n, B, 0, s>>>(L.cont, done, L.rp, L.cols, L.c16, L.cbase, L.vals, \
-                                                                    L.dinv, L.b, L.y, L.x)
+                                                                    L.dinv, L.b, L.y, L.x, H->omega)
     if (L.c16 && L.rowrel) {
       constexpr int NW = 2;
       RUV_SMOOTH_SWITCH(la, CALL)
@@ -2503,7 +2513,7 @@ int kform(Ctx& ctx, AmgHierarchy* H, const int32_t* done, int k) {
   const int la = lanes_at("RUV_AMG_LANES", k, L.n ? (double)L.nnz / (double)L.n : 1.0, smoother_lanes);
 #define CALL(X, UU, KK)                                                                                                \
   k_smooth_down<NR, X, UU, KK, NW><<<(unsigned)L.cont.n, B, 0, s>>>(L.cont, done, L.rp, L.cols, L.c16, L.cbase, L.vals, \
-                                                                    L.dinv, L.b, L.x, L.t)
+                                                                    L.dinv, L.b, L.x, L.t, kOmega)
   if (L.c16 && L.rowrel) {
     constexpr int NW = 2;
     RUV_SMOOTH_SWITCH(la, CALL)
@@ -2571,9 +2581,10 @@ namespace {
 // (FP32 rounding, the coarse over-correction), so the CG uses the flexible beta.
 class AmgPrecond final : public SepPrecond {
  public:
-  AmgPrecond(Ctx& ctx, const DevSystem& sys, bool smooth) {
+  AmgPrecond(Ctx& ctx, const DevSystem& sys, bool smooth, float omega, bool first_form) {
     std::string info;
-    H_ = amg_setup(ctx, sys, smooth, info);
+    H_ = amg_setup(ctx, sys, smooth, info, first_form);
+    H_->omega = omega;
   }
   ~AmgPrecond() override { amg_free(H_); }
   bool native_fp64() const override { return false; }
@@ -2590,6 +2601,7 @@ class AmgPrecond final : public SepPrecond {
     M.fac_off = H_->fac_off;
     M.fac = H_->fac;
     M.alpha_c = H_->alpha_c;
+    M.omega = H_->omega;
     // lanes a row needs so that each has at most a sweep of eight entries and a half
     auto lanes = [](int64_t nnz, int64_t n) {
       const double avg = n > 0 ? (double)nnz / (double)n : 1.0;
@@ -2609,8 +2621,15 @@ class AmgPrecond final : public SepPrecond {
 };
 }  // namespace
 
-std::unique_ptr<SepPrecond> make_amg(Ctx& ctx, const DevSystem& sys, bool smooth) {
-  return std::unique_ptr<SepPrecond>(new AmgPrecond(ctx, sys, smooth));
+// The smoothers' weight on a chart's Laplacian (two right-hand sides).  Its edge weights are not negative, so
+// D^-1 A has no eigenvalue above 2 and any weight below 1 damps.  Iterations (max) and time at 0.6 / 0.667 /
+// 0.75 / 0.85 / 0.92 / 0.99: 4096 disks 32 / 30 / 28 / 26 / 26 / 40, 111 / 107 / 105 / 104 / 104 / 138 ms;
+// 1024^2 field 117 / 108 / 99 / 92 / 90 / 98, 37.6 / 35.1 / 33.0 / 31.1 / 31.2 / 33.2 ms.  A system from outside may
+// have larger eigenvalues and keeps 2/3, and so does a solve that asks for the first form's sums.
+constexpr float kOmegaChart = 0.85f;
+std::unique_ptr<SepPrecond> make_amg(Ctx& ctx, const DevSystem& sys, bool smooth, bool first_form) {
+  return std::unique_ptr<SepPrecond>(
+      new AmgPrecond(ctx, sys, smooth, sys.nrhs == 2 && !first_form ? kOmegaChart : kOmega, first_form));
 }
 
 }  // namespace ruv

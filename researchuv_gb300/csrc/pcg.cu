@@ -1639,7 +1639,7 @@ std::vector<ChartResult> pcg_solve(Ctx& ctx, DevSystem& sys, double* x, const So
     } guard{e};
     RUV_CUDA(cudaEventRecord(e[0], ctx.stream));
     std::unique_ptr<SepPrecond> P = (o.precond == RUV_PRECOND_AMG || o.precond == RUV_PRECOND_AMG_SA)
-                                        ? make_amg(ctx, sys, o.precond == RUV_PRECOND_AMG_SA)
+                                        ? make_amg(ctx, sys, o.precond == RUV_PRECOND_AMG_SA, !o.teams)
                                         : make_ic0(ctx, sys, o.precond == RUV_PRECOND_IC0_COLOR);
     RUV_CUDA(cudaEventRecord(e[1], ctx.stream));
     RUV_CUDA(cudaEventSynchronize(e[1]));

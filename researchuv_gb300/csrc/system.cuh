@@ -41,7 +41,10 @@ struct SolveOpts {
   ruv_precision precision = RUV_PREC_FP64;
   double tol = 1e-12;
   int64_t max_iter = 16384;
-  bool teams = true;  // charts may be solved by the team kernels (team.cu), tiles follow the system's size
+  // false: every sum in the order, and the V-cycle with the weight, that solves had before teams, tiles by
+  // size and kOmegaChart (KeepMetric: a chart whose area iteration does not settle carries the solve's
+  // last bits into its result)
+  bool teams = true;
 };
 
 struct ChartResult {
@@ -72,7 +75,8 @@ struct SepPrecond {
 
 // Batched aggregation AMG (amg.cu): hierarchy built on the device, one V(1,1) cycle per apply.
 struct AmgHierarchy;
-AmgHierarchy* amg_setup(Ctx& ctx, const DevSystem& sys, bool smooth, std::string& info);
+// first_form: the rules that KeepMetric's solves keep (SolveOpts::teams).
+AmgHierarchy* amg_setup(Ctx& ctx, const DevSystem& sys, bool smooth, std::string& info, bool first_form);
 void amg_free(AmgHierarchy* H);
 int amg_levels(const AmgHierarchy* H);
 // One level of the hierarchy amg_setup builds for `sys`, copied to the host: its operator
@@ -90,7 +94,7 @@ struct AmgLevelHost {
 void amg_export_level(Ctx& ctx, const DevSystem& sys, bool smooth, int level, AmgLevelHost& out);
 void amg_bind(Ctx& ctx, AmgHierarchy* H, float* r0, float* z0);
 int amg_apply(Ctx& ctx, AmgHierarchy* H, const int32_t* done);
-std::unique_ptr<SepPrecond> make_amg(Ctx& ctx, const DevSystem& sys, bool smooth);
+std::unique_ptr<SepPrecond> make_amg(Ctx& ctx, const DevSystem& sys, bool smooth, bool first_form);
 
 // Batched IC(0), natural or multi-colour ordering (ic0.cu): factor on the device, two
 // level-scheduled triangular sweeps per apply.

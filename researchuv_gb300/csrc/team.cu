@@ -297,7 +297,7 @@ __device__ __forceinline__ void team_vcycle(const Team& tm, const TeamShared& sh
       level_step<NR>(
           place_of(tm, sh.lvl_n[k + 1], L.r_lanes, k + 1 >= tail), sh.lvl_row[k + 1], L.roff,
           [&](int32_t e, int32_t) { return __ldg(L.rc + e); }, [&](int32_t e) { return __ldg(L.rv + e); },
-          [&](int32_t j) { return ldv<float, NR>(L.t, j); }, [&](int32_t i) { return kTeamOmega * __ldg(C.dinv + i); },
+          [&](int32_t j) { return ldv<float, NR>(L.t, j); }, [&](int32_t i) { return M.omega * __ldg(C.dinv + i); },
           [&](int32_t i, float wd, const Vf& s) {
             stv<float, NR>(C.b, i, s);
             Vf y;
@@ -384,7 +384,7 @@ __device__ __forceinline__ void team_vcycle(const Team& tm, const TeamShared& sh
     };
     auto early = [&](int32_t i) { return Early{ldv<float, NR>(L.b, i), yval(i)}; };
     auto fin = [&](int32_t i, const Early& x, const Vf& s) {
-      const float wd = kTeamOmega * __ldg(L.dinv + i);
+      const float wd = M.omega * __ldg(L.dinv + i);
       Vf z;
 #pragma unroll
       for (int c = 0; c < NR; ++c) z.c[c] = x.b.c[c] + wd * (x.a.c[c] - s.c[c]);
@@ -574,7 +574,7 @@ __global__ void __launch_bounds__(kTeamThreads, team_per_sm<S, PCK>())
   // a row's r has its final value for the V-cycle: level 0's right-hand side and pre-smoothed values
   auto put_r = [&](int32_t i, const Vs& r) {
     if constexpr (PCK == 1) {
-      const float wd = kTeamOmega * __ldg(M.lv[0].dinv + i);
+      const float wd = M.omega * __ldg(M.lv[0].dinv + i);
       V<float, NR> t, x;
 #pragma unroll
       for (int c = 0; c < NR; ++c) {

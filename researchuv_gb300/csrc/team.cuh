@@ -27,7 +27,7 @@ struct TeamAmg {
   const int32_t* final_lvl;
   const int64_t* fac_off;
   const float* fac;
-  float alpha_c;
+  float alpha_c, omega;
   TeamLevel lv[kTeamMaxLevels];
 };
 

@@ -6,7 +6,6 @@
 
 namespace ruv {
 
-constexpr float kTeamOmega = 2.0f / 3.0f;  // the V-cycle's Jacobi weight (amg.cu kOmega)
 constexpr int kTeamDirect = 64;            // rows solved by the dense inverse (amg.cu kDirect)
 
 // 1 / d for a finite d whose reciprocal is normal: an FP32 seed of the significand and two Newton
