@@ -462,7 +462,8 @@ ruv_status ruv_amg_export(ruv_ctx* ctx, int32_t n, const int32_t* row_ptr, const
 
 namespace {
 // The batch upload.  With `overlap` (the one-call solve) the triangles and positions go in
-// parts split at chart boundaries (about equal triangle counts; RUV_UPLOAD_PARTS, default 8):
+// parts split at chart boundaries (about equal triangle counts; RUV_UPLOAD_PARTS, by default one
+// for each half million triangles, at most 8):
 // the first part on the main stream, the others and then the arrays the assembly reads only
 // after its cotangent pass (pin flags, pin targets, tangent-frame positions) on the side
 // stream, under the kernels of the parts before them.  bt.part_ready, bt.pins_ready and
@@ -503,7 +504,9 @@ ruv_status upload_batch(ruv_ctx* ctx, const ruv_lscm_batch* in, bool overlap) {
     // part k: charts [cs[k], cs[k + 1]), cs[k] the first chart boundary at or past k / P of
     // the triangles
     const char* parts_env = std::getenv("RUV_UPLOAD_PARTS");
-    const int env_parts = parts_env ? std::atoi(parts_env) : 8;
+    // (a part's kernels take 20 us however few triangles it has.  Assembly in 8 parts / one: 600
+    // triangles 0.21 / 0.12 ms, 32,000 0.32 / 0.165; a half million take longer to copy than to assemble)
+    const int env_parts = parts_env ? std::atoi(parts_env) : (int)std::min<int64_t>(8, 1 + NT / 500000);
     const int P = overlap ? (int)std::max<int64_t>(1, std::min<int64_t>({(int64_t)env_parts, DevBatch::kMaxParts, NC}))
                           : 1;
     std::vector<int64_t> cs(P + 1, NC);
