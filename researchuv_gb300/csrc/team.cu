@@ -951,7 +951,15 @@ int64_t team_solve(Ctx& ctx, const DevSystem& sys, const TeamLoop<S>& loop, cons
   int64_t left = 0, largest = 0;
   for (int64_t c = 0; c < NC; ++c) largest = std::max(largest, rows_of(c));
   const char* re = std::getenv("RUV_TEAM_ROWS");
-  const int64_t most = re ? std::atoll(re) : mixed ? 131072 : 40000;
+  // The largest chart a team of 16 SMs takes, where both ways were measured (ms, team / launch loop):
+  // mixed Jacobi 39,000 rows 21.8 / 31.9, 89,000 57 / 60, 128,000 121 / 102; FP64 Jacobi, two columns,
+  // 19,000 rows 16.2 / 19.4, 39,000 37 / 27, one column half the arithmetic; V-cycle 32,000 rows mixed
+  // 5.8 / 6.4, FP64 6.2 / 6.6, 89,000 mixed 11.9 / 9.4; colour-ordered IC(0) 14,400 rows 7.0 / 35.
+  const int64_t most = re                ? std::atoll(re)
+                       : kind == 1       ? (mixed ? 40000 : 32000)
+                       : kind == 2       ? (mixed ? 90000 : 40000)
+                       : mixed           ? 90000
+                                         : 48000 / NR;
   // a V-cycle is a chain of small steps, and a chart left to the other loop makes them all again: all
   // charts by teams, or none.  Teams hold 512 rows in flight on an SM where the launch loop's kernels
   // stream: 473,000 rows in 300 charts took 146 us an iteration against 172, 14.4 million 7,000 against
