@@ -34,6 +34,9 @@ namespace ruv {
 namespace {
 
 constexpr int kAmgThreads = 256;
+// groups up to which the group graph takes a warp for each (us, warp / thread: 900 groups 9 / 199,
+// 4,600 21 / 100, 36,000 43 / 50; 204,000 groups take a thread each 37 us)
+constexpr int64_t kGroupWarps = 65536;
 constexpr int kDirect = 64;       // rows at which a chart is solved directly
 constexpr int kMaxLevels = 16;
 constexpr float kOmega = 2.0f / 3.0f;
@@ -176,6 +179,31 @@ __device__ __forceinline__ uint32_t pair_priority(int32_t i, int32_t j) {
 // proposals likely even where couplings vary monotonically along a row of the mesh (a
 // weight-ordered handshake then chains i -> i-1 -> i-2 ... and pairs almost nothing).
 constexpr float kStrong = 0.85f;
+
+// fn(column, map[column], value) over the entries [beg, end) of a row, in order, eight loads of
+// each array in flight: these kernels wait on their loads (one row a thread, entry by entry, took a
+// level of 92,000 rows 13.5 us for a round of k_propose).
+template <class Fn>
+__device__ __forceinline__ void walk_entries(int beg, int end, const int32_t* __restrict__ cols,
+                                             const float* __restrict__ vals, const int32_t* __restrict__ map, Fn fn) {
+  constexpr int U = 8;
+  for (int e = beg; e < end; e += U) {
+    int32_t j[U], h[U];
+    float v[U];
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      const int x = min(e + q, end - 1);
+      j[q] = cols[x];
+      v[q] = vals[x];
+    }
+#pragma unroll
+    for (int q = 0; q < U; ++q) h[q] = map[j[q]];
+#pragma unroll
+    for (int q = 0; q < U; ++q)
+      if (e + q < end) fn(j[q], h[q], v[q]);
+  }
+}
+
 __global__ void k_propose(int64_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ cols,
                           const float* __restrict__ vals, const uint8_t* __restrict__ active,
                           const int32_t* __restrict__ mate, int32_t* __restrict__ prop, float strong) {
@@ -183,21 +211,21 @@ __global__ void k_propose(int64_t n, const int32_t* __restrict__ rp, const int32
   if (i >= n) return;
   int32_t best = -1;
   if (active[i] && mate[i] < 0) {
+    const int beg = rp[i], end = rp[i + 1];
     float mx = 0.0f;
-    for (int e = rp[i]; e < rp[i + 1]; ++e) {
-      const int32_t j = cols[e];
-      if (j != i && mate[j] < 0) mx = fmaxf(mx, fabsf(vals[e]));
-    }
+    walk_entries(beg, end, cols, vals, mate, [&](int32_t j, int32_t mj, float v) {
+      if (j != i && mj < 0) mx = fmaxf(mx, fabsf(v));
+    });
     uint32_t bp = 0;
-    for (int e = rp[i]; e < rp[i + 1]; ++e) {
-      const int32_t j = cols[e];
-      if (j == i || mate[j] >= 0 || !(fabsf(vals[e]) >= strong * mx) || mx == 0.0f) continue;
-      const uint32_t pr = pair_priority((int32_t)i, j);
-      if (best < 0 || pr > bp || (pr == bp && j < best)) {
-        bp = pr;
-        best = j;
-      }
-    }
+    if (mx != 0.0f)
+      walk_entries(beg, end, cols, vals, mate, [&](int32_t j, int32_t mj, float v) {
+        if (j == i || mj >= 0 || !(fabsf(v) >= strong * mx)) return;
+        const uint32_t pr = pair_priority((int32_t)i, j);
+        if (best < 0 || pr > bp || (pr == bp && j < best)) {
+          bp = pr;
+          best = j;
+        }
+      });
   }
   prop[i] = best;
 }
@@ -356,10 +384,9 @@ __global__ void k_group_graph(int64_t ng, const int64_t* __restrict__ goff, cons
   int n = 0;
   for (int64_t a = goff[g]; a < goff[g + 1]; ++a) {
     const int32_t i = mem[a];
-    for (int e = rp[i]; e < rp[i + 1]; ++e) {
-      const int32_t h = grp_of[cols[e]];
-      if (h == (int32_t)g) continue;
-      const float v = fabsf(vals[e]);
+    walk_entries(rp[i], rp[i + 1], cols, vals, grp_of, [&](int32_t, int32_t h, float w) {
+      if (h == (int32_t)g) return;
+      const float v = fabsf(w);
       bool hit = false;
 #pragma unroll
       for (int t = 0; t < kReg; ++t)
@@ -367,7 +394,7 @@ __global__ void k_group_graph(int64_t ng, const int64_t* __restrict__ goff, cons
           rv[t] += v;
           hit = true;
         }
-      if (hit) continue;
+      if (hit) return;
       int t = kReg;
       while (t < n && K[t] != h) ++t;
       if (t < n) {
@@ -385,7 +412,7 @@ __global__ void k_group_graph(int64_t ng, const int64_t* __restrict__ goff, cons
         V[n] = v;
         ++n;
       }
-    }
+    });
   }
 #pragma unroll
   for (int t = 0; t < kReg; ++t)
@@ -394,6 +421,82 @@ __global__ void k_group_graph(int64_t ng, const int64_t* __restrict__ goff, cons
       V[t] = rv[t];
     }
   gn[g] = n;
+}
+
+// k_group_graph with a warp per group, for levels of few groups: a thread's chain of dependent
+// loads and key comparisons, not the chip, sets the time there, and it grows with the denser rows of
+// the coarse levels.  32 entries are loaded at once and taken in order by the whole warp, key t (of
+// the first 64) held by lane t mod 32, the rest in the row's global area: the same keys in the same
+// order, each strength summed in the same order.
+__global__ void k_group_graph_warp(int64_t ng, const int64_t* __restrict__ goff, const int32_t* __restrict__ mem,
+                                   const int32_t* __restrict__ rp, const int32_t* __restrict__ cols,
+                                   const float* __restrict__ vals, const int32_t* __restrict__ grp_of,
+                                   const int64_t* __restrict__ gcap_off, int32_t* __restrict__ gn, int32_t* gkey,
+                                   float* gval) {
+  const int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (g >= ng) return;  // (the whole warp)
+  const int lane = threadIdx.x & 31;
+  int32_t* K = gkey + gcap_off[g];
+  float* V = gval + gcap_off[g];
+  int32_t k0 = -1, k1 = -1;
+  float v0 = 0.0f, v1 = 0.0f;
+  int n = 0;
+  for (int64_t a = goff[g]; a < goff[g + 1]; ++a) {
+    const int32_t i = mem[a];
+    const int end = rp[i + 1];
+    for (int e0 = rp[i]; e0 < end; e0 += 32) {
+      const int e = min(e0 + lane, end - 1);
+      const int32_t h = grp_of[cols[e]];
+      const float v = fabsf(vals[e]);
+      const int cnt = min(32, end - e0);
+      for (int q = 0; q < cnt; ++q) {
+        const int32_t hq = __shfl_sync(0xffffffffu, h, q);
+        const float vq = __shfl_sync(0xffffffffu, v, q);
+        if (hq == (int32_t)g) continue;
+        const bool mine0 = k0 == hq, mine1 = k1 == hq;
+        if (__any_sync(0xffffffffu, mine0 || mine1)) {
+          if (mine0) v0 += vq;
+          if (mine1) v1 += vq;
+        } else if (n < 64) {
+          if (lane == (n & 31)) {
+            if (n < 32) {
+              k0 = hq;
+              v0 = vq;
+            } else {
+              k1 = hq;
+              v1 = vq;
+            }
+          }
+          ++n;
+        } else {
+          int at = -1;
+          for (int t = 64; t < n && at < 0; t += 32) {
+            const unsigned f = __ballot_sync(0xffffffffu, t + lane < n && K[t + lane] == hq);
+            if (f) at = t + __ffs(f) - 1;
+          }
+          if (lane == 0) {
+            if (at >= 0) {
+              V[at] += vq;
+            } else {
+              K[n] = hq;
+              V[n] = vq;
+            }
+          }
+          if (at < 0) ++n;
+          __syncwarp();
+        }
+      }
+    }
+  }
+  if (lane < n) {
+    K[lane] = k0;
+    V[lane] = v0;
+  }
+  if (lane + 32 < n) {
+    K[lane + 32] = k1;
+    V[lane + 32] = v1;
+  }
+  if (lane == 0) gn[g] = n;
 }
 
 // k_propose2 over the stored group graph.
@@ -409,27 +512,26 @@ __global__ void k_propose2_graph(int64_t ng, const int64_t* __restrict__ gcap_of
     const float* V = gval + gcap_off[g];
     const int n = gn[g];
     float mx = 0.0f;
-    int kept = 0, t_end = n;
-    for (int t = 0; t < n; ++t) {
-      if (gmate[K[t]] >= 0) continue;
-      if (kept == kAccCap) {
-        t_end = t;
-        break;
-      }
+    int kept = 0;
+    walk_entries(0, n, K, V, gmate, [&](int32_t, int32_t mh, float v) {
+      if (mh >= 0 || kept == kAccCap) return;
       ++kept;
-      mx = fmaxf(mx, V[t]);
-    }
+      mx = fmaxf(mx, v);
+    });
     warp_atomic_max(stats + 2, kept);
     uint32_t bp = 0;
-    for (int t = 0; t < t_end; ++t) {
-      if (gmate[K[t]] >= 0) continue;
-      if (!(V[t] >= strong * mx) || mx == 0.0f) continue;
-      const uint32_t pr = pair_priority((int32_t)g, K[t]);
-      if (best < 0 || pr > bp || (pr == bp && K[t] < best)) {
-        bp = pr;
-        best = K[t];
-      }
-    }
+    int seen = 0;
+    if (mx != 0.0f)
+      walk_entries(0, n, K, V, gmate, [&](int32_t h, int32_t mh, float v) {
+        if (mh >= 0 || seen == kAccCap) return;
+        ++seen;
+        if (!(v >= strong * mx)) return;
+        const uint32_t pr = pair_priority((int32_t)g, h);
+        if (best < 0 || pr > bp || (pr == bp && h < best)) {
+          bp = pr;
+          best = h;
+        }
+      });
   }
   prop[g] = best;
 }
@@ -451,14 +553,14 @@ __global__ void k_group_lead_graph(int64_t ng, const int64_t* __restrict__ gcap_
     int32_t best = -1;
     float bs = -1.0f;
     int kept = 0;
-    for (int t = 0; t < n && kept < kAccCap; ++t) {
-      if (gmate[K[t]] < 0) continue;
+    walk_entries(0, n, K, V, gmate, [&](int32_t h, int32_t mh, float v) {
+      if (mh < 0 || kept == kAccCap) return;
       ++kept;
-      if (V[t] > bs || (V[t] == bs && K[t] < best)) {
-        bs = V[t];
-        best = K[t];
+      if (v > bs || (v == bs && h < best)) {
+        bs = v;
+        best = h;
       }
-    }
+    });
     L = best >= 0 ? min(best, gmate[best]) : (int32_t)g;
   }
   glead_of[g] = L;
@@ -972,8 +1074,7 @@ __global__ void k_agg_lead_rows(int64_t n, const uint8_t* __restrict__ lead, con
 // memory: Cholesky A = L L^T, then Y = L^-1, then A^-1 = Y^T Y, stored as FP32 (symmetric,
 // row-major m x m).  The V-cycle's coarse solve is then one dense mat-vec per chart instead
 // of two serial triangular sweeps.
-constexpr int kFactorThreads = 128;
-constexpr size_t kFactorSmem = 2 * sizeof(float2) * kDirect * kDirect;
+constexpr int kFactorThreads = 256;
 
 // df helpers of the dense factors: a - b, a / b and sqrt(a) on (hi, lo) pairs (one Newton
 // correction each on the FP32 quotient / root, the residual formed with error-free products)
@@ -998,6 +1099,14 @@ __device__ __forceinline__ float2 df_sqrt(float2 a) {
 // 1e10: a long chain pinned at its ends) the smallest eigenvalue of the coarse block is below
 // the rounding of its entries; the floor 1e-6 |a_jj| keeps the factor real and leaves that
 // one mode to the outer Krylov iteration.  A zero or non-finite pivot sets *bad.
+//
+// Both sweeps go in one pass of m steps over one lower triangle W: after step j its columns
+// 0 .. j hold Y and the others the trailing block.  With Z_k = Y_jk (k <= j) and L_kj (k > j),
+// step j is W_ik = (k == j ? 0 : W_ik) - Z_i Z_k for the rows i > j.  W stays in registers --
+// warp w holds the rows w + 8 q and 63 - w - 8 q, lane l their columns l and l + 32, so the
+// warps' loads stay level as the rows finish -- and a step costs two barriers, one to publish
+// its column and one to publish Z.  (W and Y in shared memory, L first and then Y, a barrier
+// more each step: 238 us for 300 blocks of up to 64 rows, now 100; 4,096 blocks 828, now 436.)
 __global__ void __launch_bounds__(kFactorThreads) k_direct_factor(const int32_t* __restrict__ final_lvl,
                                                                   const int64_t* const* __restrict__ lvl_chart_row,
                                                                   const int32_t* const* __restrict__ lvl_rp,
@@ -1005,80 +1114,118 @@ __global__ void __launch_bounds__(kFactorThreads) k_direct_factor(const int32_t*
                                                                   const double* const* __restrict__ lvl_vals,
                                                                   const int64_t* __restrict__ fac_off, float* __restrict__ fac,
                                                                   int* __restrict__ bad) {
-  extern __shared__ float2 dsm[];
-  float2* M = dsm;                      // m x m, row-major: the lower triangle becomes L
-  float2* Y = dsm + kDirect * kDirect;  // starts as I; row i becomes (L^-1)[i] at step i
-  __shared__ float dg0[kDirect];        // |a_jj| before the factorisation (the pivot floor)
+  static_assert(kDirect == 64 && kFactorThreads == 256, "the split of the triangle");
+  constexpr int kQ = 4;
+  __shared__ float2 S[kDirect * kDirect];  // A's block, then Y (its lower triangle)
+  __shared__ float2 R[kDirect];            // row j up to the diagonal and column j below it, before step j
+  __shared__ float2 Z[kDirect];
+  __shared__ float dg0[kDirect];  // |a_jj| before the factorisation (the pivot floor)
   const int c = blockIdx.x;
   const int f = final_lvl[c];
   if (f < 0) return;
   const int64_t r0 = lvl_chart_row[f][c];
   const int m = (int)(lvl_chart_row[f][c + 1] - r0);
   if (m <= 0 || m > kDirect) return;
-  for (int t = threadIdx.x; t < m * m; t += blockDim.x) {
-    M[t] = make_float2(0.0f, 0.0f);
-    Y[t] = make_float2((t / m) == (t % m) ? 1.0f : 0.0f, 0.0f);
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  const float2 zero = make_float2(0.0f, 0.0f);
+  for (int t = tid; t < kDirect * kDirect; t += kFactorThreads) S[t] = zero;
+  if (tid < kDirect) {
+    Z[tid] = zero;
+    dg0[tid] = 0.0f;
   }
-  for (int t = threadIdx.x; t < m; t += blockDim.x) dg0[t] = 0.0f;
   __syncthreads();
-  for (int r = threadIdx.x; r < m; r += blockDim.x) {
+  for (int r = tid >> 2; r < m; r += kFactorThreads >> 2) {  // four lanes per row
     const int64_t row = r0 + r;
-    for (int e = lvl_rp[f][row]; e < lvl_rp[f][row + 1]; ++e) {
+    for (int e = lvl_rp[f][row] + (tid & 3); e < lvl_rp[f][row + 1]; e += 4) {
       const int64_t col = lvl_cols[f][e] - r0;
       if (col >= 0 && col < m) {
         const double v = lvl_vals[f][e];
         const float hi = (float)v;
-        M[r * m + col] = make_float2(hi, (float)(v - (double)hi));
+        S[r * kDirect + col] = make_float2(hi, (float)(v - (double)hi));
         if (col == r) dg0[r] = fabsf(hi);
       }
     }
   }
   __syncthreads();
-  // L: column j scaled by its pivot, then the trailing block updated (entries in parallel)
+  float2 lo[kQ], hi[kQ][2];  // rows w + 8 q (columns < 32), rows 63 - w - 8 q
+#pragma unroll
+  for (int q = 0; q < kQ; ++q) {
+    lo[q] = S[(w + 8 * q) * kDirect + lane];
+    hi[q][0] = S[(63 - w - 8 * q) * kDirect + lane];
+    hi[q][1] = S[(63 - w - 8 * q) * kDirect + 32 + lane];
+  }
+  auto publish = [&](int j) {
+#pragma unroll
+    for (int q = 0; q < kQ; ++q) {
+      const int il = w + 8 * q, ih = 63 - w - 8 * q;
+      if (il >= j && il < m && lane == j) R[il] = lo[q];
+      if (il == j && lane < j) R[lane] = lo[q];
+      if (ih >= j && ih < m && lane == (j & 31)) R[ih] = j < 32 ? hi[q][0] : hi[q][1];
+      if (ih == j) {
+        if (lane < j) R[lane] = hi[q][0];
+        if (lane + 32 < j) R[lane + 32] = hi[q][1];
+      }
+    }
+  };
+  publish(0);
   for (int j = 0; j < m; ++j) {
-    if (threadIdx.x == 0) {
-      float2 d = M[j * m + j];
+    __syncthreads();
+    if (tid < m) {
+      float2 d = R[j];
       const float fl = 1e-6f * dg0[j];
       if (!(d.x > fl)) d = make_float2(fl, 0.0f);
       if (!(d.x > 0.0f) || !isfinite(d.x)) {  // a zero or non-finite diagonal
-        atomicExch(bad, 1);
+        if (tid == 0) atomicExch(bad, 1);
         d = make_float2(1e-30f, 0.0f);
       }
-      M[j * m + j] = df_sqrt(d);
+      const float2 z = df_div(tid == j ? make_float2(1.0f, 0.0f) : R[tid], df_sqrt(d));
+      Z[tid] = z;
+      if (tid <= j) S[j * kDirect + tid] = z;
     }
     __syncthreads();
-    const float2 piv = M[j * m + j];
-    for (int i = j + 1 + threadIdx.x; i < m; i += blockDim.x) M[i * m + j] = df_div(M[i * m + j], piv);
-    __syncthreads();
-    const int w = m - j - 1;  // trailing block: rows and columns j+1 .. m-1, lower triangle
-    for (int t = threadIdx.x; t < w * w; t += blockDim.x) {
-      const int i = j + 1 + t / w, k = j + 1 + t % w;
-      if (k > i) continue;
-      M[i * m + k] = df_add(M[i * m + k], df_neg(df_mul(M[i * m + j], M[k * m + j])));
+    const float2 z0 = Z[lane], z1 = Z[lane + 32];
+#pragma unroll
+    for (int q = 0; q < kQ; ++q) {
+      const int il = w + 8 * q, ih = 63 - w - 8 * q;
+      if (il > j && il < m) lo[q] = df_add(lane == j ? zero : lo[q], df_neg(df_mul(Z[il], z0)));
+      if (ih > j && ih < m) {
+        const float2 zi = Z[ih];
+        hi[q][0] = df_add(lane == j ? zero : hi[q][0], df_neg(df_mul(zi, z0)));
+        hi[q][1] = df_add(lane + 32 == j ? zero : hi[q][1], df_neg(df_mul(zi, z1)));
+      }
     }
-    __syncthreads();
+    if (j + 1 < m) publish(j + 1);
   }
-  // Y = L^-1: row i scaled by L_ii, then the rows below updated
-  for (int i = 0; i < m; ++i) {
-    const float2 lii = M[i * m + i];
-    for (int j = threadIdx.x; j <= i; j += blockDim.x) Y[i * m + j] = df_div(Y[i * m + j], lii);
-    __syncthreads();
-    const int rows = m - i - 1;
-    for (int t = threadIdx.x; t < rows * (i + 1); t += blockDim.x) {
-      const int k = i + 1 + t / (i + 1), j = t % (i + 1);
-      Y[k * m + j] = df_add(Y[k * m + j], df_neg(df_mul(M[k * m + i], Y[i * m + j])));
+  __syncthreads();
+  // A^-1 = Y^T Y: (A^-1)[i][k] = sum_{j >= k} Y[j][i] Y[j][k], i <= k and mirrored; the same split,
+  // k the row, i the column
+#pragma unroll
+  for (int q = 0; q < kQ; ++q) lo[q] = hi[q][0] = hi[q][1] = zero;
+  for (int j = w; j < m; ++j) {
+    const float2 y0 = S[j * kDirect + lane], y1 = S[j * kDirect + 32 + lane];
+#pragma unroll
+    for (int q = 0; q < kQ; ++q) {
+      const int il = w + 8 * q, ih = 63 - w - 8 * q;
+      if (il <= j) lo[q] = df_add(lo[q], df_mul(y0, S[j * kDirect + il]));
+      if (ih <= j) {
+        const float2 yk = S[j * kDirect + ih];
+        hi[q][0] = df_add(hi[q][0], df_mul(y0, yk));
+        hi[q][1] = df_add(hi[q][1], df_mul(y1, yk));
+      }
     }
-    __syncthreads();
   }
-  // A^-1 = Y^T Y: (A^-1)[i][k] = sum_{j >= max(i,k)} Y[j][i] Y[j][k], for i <= k and mirrored
   float* Ainv = fac + fac_off[c];
-  for (int t = threadIdx.x; t < m * m; t += blockDim.x) {
-    const int i = t / m, k = t % m;
-    if (i > k) continue;
-    float2 s = make_float2(0.0f, 0.0f);
-    for (int j = k; j < m; ++j) s = df_add(s, df_mul(Y[j * m + i], Y[j * m + k]));
-    Ainv[i * m + k] = s.x;
-    Ainv[k * m + i] = s.x;
+  auto store = [&](int i, int k, float v) {
+    if (k < m && i <= k) {
+      Ainv[i * m + k] = v;
+      Ainv[k * m + i] = v;
+    }
+  };
+#pragma unroll
+  for (int q = 0; q < kQ; ++q) {
+    store(lane, w + 8 * q, lo[q].x);
+    store(lane, 63 - w - 8 * q, hi[q][0].x);
+    store(lane + 32, 63 - w - 8 * q, hi[q][1].x);
   }
 }
 
@@ -1582,15 +1729,19 @@ __global__ void __launch_bounds__(kAmgThreads) k_smooth_up_t(LvlTiles T, const i
 }
 
 // Direct solve of every chart at its last level: x = A^-1 b with the dense inverse (one CTA
-// of kDirect threads per chart, thread i forms row i; A^-1 is symmetric, so row i is read as
-// column i and the loads coalesce across threads).
+// per chart).  The whole inverse is brought to shared memory by all threads at once, then thread i
+// forms row i (read as column i: A^-1 is symmetric) in column order: one trip to L2, where loads
+// inside the sum took four (one chart of 64 rows 11.5 us a call, now 4.7).
+constexpr int kDirectThreads = 256;
 template <int NR>
-__global__ void __launch_bounds__(kDirect) k_direct_solve(const int32_t* __restrict__ final_lvl, const int32_t* __restrict__ done,
+__global__ void __launch_bounds__(kDirectThreads) k_direct_solve(const int32_t* __restrict__ final_lvl,
+                                                          const int32_t* __restrict__ done,
                                                           const int64_t* const* __restrict__ lvl_chart_row,
                                                           float* const* __restrict__ lvl_b, float* const* __restrict__ lvl_x,
                                                           const float* const* __restrict__ lvl_dinv,
                                                           const int64_t* __restrict__ fac_off, const float* __restrict__ fac,
                                                           int lo, int hi) {
+  __shared__ float As[kDirect * kDirect];
   __shared__ float bs[NR][kDirect];
   const int c = blockIdx.x;
   const int f = final_lvl[c];
@@ -1608,26 +1759,27 @@ __global__ void __launch_bounds__(kDirect) k_direct_solve(const int32_t* __restr
       for (int k = 0; k < NR; ++k) x[NR * (r0 + r) + k] = dv[r0 + r] * b[NR * (r0 + r) + k];
     return;
   }
+  const float* Ainv = fac + fac_off[c];
+  float a[kDirect * kDirect / kDirectThreads];
+#pragma unroll
+  for (int q = 0; q < kDirect * kDirect / kDirectThreads; ++q) {
+    const int t = i + q * kDirectThreads;
+    a[q] = t < m * m ? __ldg(Ainv + t) : 0.0f;
+  }
   if (i < m)
 #pragma unroll
     for (int k = 0; k < NR; ++k) bs[k][i] = b[NR * (r0 + i) + k];
+#pragma unroll
+  for (int q = 0; q < kDirect * kDirect / kDirectThreads; ++q) As[i + q * kDirectThreads] = a[q];
   __syncthreads();
   if (i >= m) return;
-  const float* Ainv = fac + fac_off[c];
   float s[NR];
 #pragma unroll
   for (int k = 0; k < NR; ++k) s[k] = 0.0f;
-  // (sixteen columns loaded at a time, added in order: one load in flight took 14 us for one chart)
-  for (int j0 = 0; j0 < m; j0 += 16) {
-    float a[16];
+#pragma unroll 16
+  for (int j = 0; j < m; ++j)
 #pragma unroll
-    for (int q = 0; q < 16; ++q) a[q] = j0 + q < m ? __ldg(Ainv + (j0 + q) * m + i) : 0.0f;
-#pragma unroll
-    for (int q = 0; q < 16; ++q)
-      if (j0 + q < m)
-#pragma unroll
-        for (int k = 0; k < NR; ++k) s[k] += a[q] * bs[k][j0 + q];
-  }
+    for (int k = 0; k < NR; ++k) s[k] += As[j * m + i] * bs[k][j];
 #pragma unroll
   for (int k = 0; k < NR; ++k) x[NR * (r0 + i) + k] = s[k];
 }
@@ -2007,7 +2159,11 @@ AmgHierarchy* amg_setup(Ctx& ctx, const DevSystem& sys, bool smooth, std::string
         const int64_t GE = read_i64(ctx, gcap_off + NG);
         int32_t* gkey = ctx.ws.get<int32_t>("amg.gkey", std::max<int64_t>(GE, 1));
         float* gval = ctx.ws.get<float>("amg.gval", std::max<int64_t>(GE, 1));
-        k_group_graph<<<div_up(NG, B), B, 0, s>>>(NG, goff, mem, L.rp, L.cols, L.vals, grp_of, gcap_off, gn, gkey, gval);
+        if (NG <= kGroupWarps)
+          k_group_graph_warp<<<div_up(32 * NG, B), B, 0, s>>>(NG, goff, mem, L.rp, L.cols, L.vals, grp_of, gcap_off, gn, gkey,
+                                                              gval);
+        else
+          k_group_graph<<<div_up(NG, B), B, 0, s>>>(NG, goff, mem, L.rp, L.cols, L.vals, grp_of, gcap_off, gn, gkey, gval);
         count_launches(1);
         for (int r = 0; r < rounds; ++r) {
           k_propose2_graph<<<div_up(NG, B), B, 0, s>>>(NG, gcap_off, gn, gkey, gval, gmate, gprop, ovf, strong);
@@ -2239,8 +2395,7 @@ AmgHierarchy* amg_setup(Ctx& ctx, const DevSystem& sys, bool smooth, std::string
   RUV_CUDA(cudaMemcpyAsync(H->d_lvl_dinv, dvs.data(), sizeof(void*) * K, cudaMemcpyHostToDevice, s));
   int* bad = ovf + 1;
   if (NC > 0) {
-    RUV_CUDA(cudaFuncSetAttribute(k_direct_factor, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFactorSmem));
-    k_direct_factor<<<(unsigned)NC, kFactorThreads, kFactorSmem, s>>>(H->final_lvl, H->d_lvl_chart_row, d_rp, d_cols, d_vals, H->fac_off,
+    k_direct_factor<<<(unsigned)NC, kFactorThreads, 0, s>>>(H->final_lvl, H->d_lvl_chart_row, d_rp, d_cols, d_vals, H->fac_off,
                                                  H->fac, bad);
     count_launches(1);
   }
@@ -2440,7 +2595,7 @@ int vtail(Ctx& ctx, AmgHierarchy* H, const int32_t* done, int k0) {
 #undef CALL
     ++launches;
   }
-  k_direct_solve<NR><<<(unsigned)H->n_charts, kDirect, 0, s>>>(H->final_lvl, done, H->d_lvl_chart_row, H->d_lvl_b,
+  k_direct_solve<NR><<<(unsigned)H->n_charts, kDirectThreads, 0, s>>>(H->final_lvl, done, H->d_lvl_chart_row, H->d_lvl_b,
                                                                H->d_lvl_x, H->d_lvl_dinv, H->fac_off, H->fac, k0, kMaxLevels);
   ++launches;
   for (int k = K - 2; k >= k0; --k) {
@@ -2556,7 +2711,7 @@ int kform(Ctx& ctx, AmgHierarchy* H, const int32_t* done, int k) {
     k_kupdate<NR><<<(unsigned)L.cont.n, B, 0, s>>>(L.cont, done, L.kbeta, L.y, L.w, L.x, step == 0 ? L.t : nullptr);
     launches += 4;
   }
-  k_direct_solve<NR><<<(unsigned)H->n_charts, kDirect, 0, s>>>(H->final_lvl, done, H->d_lvl_chart_row, H->d_lvl_b,
+  k_direct_solve<NR><<<(unsigned)H->n_charts, kDirectThreads, 0, s>>>(H->final_lvl, done, H->d_lvl_chart_row, H->d_lvl_b,
                                                                H->d_lvl_x, H->d_lvl_dinv, H->fac_off, H->fac, k, k);
   return launches + 1;
 }
