@@ -410,36 +410,71 @@ __global__ void k_driver_state_init(DriverState* st, int64_t n_charts) {
   if (c < n_charts) st[c] = DriverState{1.0, __longlong_as_double(0x7ff0000000000000ll), 1.0, 0, 1, 0};
 }
 
-__device__ __forceinline__ void new_uv_of(int64_t v, const uint8_t* pinned, const double* pin_uv, const int64_t* row_of,
-                                          const double* x, double& u, double& w) {
-  if (pinned[v]) {
-    u = pin_uv[2 * v];
-    w = pin_uv[2 * v + 1];
-  } else {
-    int64_t r = row_of[v];
-    u = x[2 * r];
-    w = x[2 * r + 1];
+// The solution the driver moves to: the solve's x, or KeepMetric's x = y_b - aux y_u.
+struct DriverX {
+  const double* x;   // (y_b for KeepMetric)
+  const double* yu;  // null: plain x
+  const double* aux; // per chart
+};
+
+// fn(v, new u, new v, uv) of the vertices beg + thread, + blockDim, ... below end, in that order, the loads
+// of U vertices in flight at once: a thread's vertices one after another, a chain of three loads each,
+// took 9.4 us a launch for 32 charts of up to 3,000 vertices.
+template <bool KEEP, int U, class Fn>
+__device__ __forceinline__ void driver_verts(int64_t beg, int64_t end, const uint8_t* __restrict__ pinned,
+                                             const double* __restrict__ pin_uv, const int64_t* __restrict__ row_of,
+                                             const DriverX& X, double aux, const double* uv, Fn fn) {
+  for (int64_t v0 = beg + threadIdx.x; v0 < end; v0 += (int64_t)U * blockDim.x) {
+    const double* p[U];
+    const double* py[U];
+    double nu[U], nw[U], ou[U], ow[U];
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      const int64_t v = min(v0 + (int64_t)q * blockDim.x, end - 1);
+      const bool pin = pinned[v];
+      const int64_t r = row_of[v];
+      p[q] = pin ? pin_uv + 2 * v : X.x + 2 * r;
+      py[q] = KEEP && !pin ? X.yu + 2 * r : nullptr;
+      ou[q] = uv[2 * v];
+      ow[q] = uv[2 * v + 1];
+    }
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      nu[q] = p[q][0];
+      nw[q] = p[q][1];
+      if (KEEP && py[q] != nullptr) {
+        nu[q] = nu[q] - aux * py[q][0];
+        nw[q] = nw[q] - aux * py[q][1];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      const int64_t v = v0 + (int64_t)q * blockDim.x;
+      if (v < end) fn(v, nu[q], nw[q], ou[q], ow[q]);
+    }
   }
 }
 
 // per vertex-tile partial sums of |new_uv - uv|^2 and |uv|^2 for active charts
-__global__ void k_driver_partials(const int64_t* __restrict__ tile_beg, const int32_t* __restrict__ tile_chart,
-                                  int64_t n_tiles, const DriverState* __restrict__ st, const uint8_t* __restrict__ pinned,
-                                  const double* __restrict__ pin_uv, const int64_t* __restrict__ row_of,
-                                  const double* __restrict__ x, const double* __restrict__ uv,
-                                  double* __restrict__ part) {
+template <bool KEEP>
+__global__ void __launch_bounds__(256) k_driver_partials(const int64_t* __restrict__ tile_beg,
+                                                         const int32_t* __restrict__ tile_chart,
+                                                         const DriverState* __restrict__ st,
+                                                         const uint8_t* __restrict__ pinned,
+                                                         const double* __restrict__ pin_uv,
+                                                         const int64_t* __restrict__ row_of, DriverX X,
+                                                         const double* __restrict__ uv, double* __restrict__ part) {
   __shared__ double sh[64];
   int64_t t = blockIdx.x;
   int c = tile_chart[t];
-  if (!st[c].active) return;
+  if (st[c].active != 1) return;
   double s[2] = {0.0, 0.0};
-  for (int64_t v = tile_beg[2 * t] + threadIdx.x; v < tile_beg[2 * t + 1]; v += blockDim.x) {
-    double nu, nw;
-    new_uv_of(v, pinned, pin_uv, row_of, x, nu, nw);
-    double du = nu - uv[2 * v], dw = nw - uv[2 * v + 1];
-    s[0] += du * du + dw * dw;
-    s[1] += uv[2 * v] * uv[2 * v] + uv[2 * v + 1] * uv[2 * v + 1];
-  }
+  driver_verts<KEEP, 4>(tile_beg[2 * t], tile_beg[2 * t + 1], pinned, pin_uv, row_of, X, KEEP ? X.aux[c] : 0.0, uv,
+                        [&](int64_t, double nu, double nw, double ou, double ow) {
+                          double du = nu - ou, dw = nw - ow;
+                          s[0] += du * du + dw * dw;
+                          s[1] += ou * ou + ow * ow;
+                        });
   block_sum<2>(s, sh);
   if (threadIdx.x == 0) {
     part[2 * t] = s[0];
@@ -451,7 +486,7 @@ __global__ void k_driver_decide(const int64_t* __restrict__ chart_tile, int64_t 
                                 const double* __restrict__ part, int it, int max_iter, int* __restrict__ n_active) {
   __shared__ double sh[64];
   int64_t c = blockIdx.x;
-  if (!st[c].active) return;
+  if (st[c].active != 1) return;
   double s[2] = {0.0, 0.0};
   for (int64_t t = chart_tile[c] + threadIdx.x; t < chart_tile[c + 1]; t += blockDim.x) {
     s[0] += part[2 * t];
@@ -473,33 +508,30 @@ __global__ void k_driver_decide(const int64_t* __restrict__ chart_tile, int64_t 
   } else {
     d.prev_err = applied;
     d.err_accum += err;
-    if (max_iter * 10 < it || it + 1 >= max_iter) d.active = 2;  // apply this update, then stop
+    if (max_iter * 10 < it || it + 1 >= max_iter) d.active = 2;  // apply this update, then stop: iteration d.iters - 1 only
   }
   st[c] = d;
   if (d.active != 1) atomicSub(n_active, 1);
 }
 
-__global__ void k_driver_apply(const int64_t* __restrict__ tile_beg, const int32_t* __restrict__ tile_chart,
-                               int64_t n_tiles, DriverState* __restrict__ st, const uint8_t* __restrict__ pinned,
-                               const double* __restrict__ pin_uv, const int64_t* __restrict__ row_of,
-                               const double* __restrict__ x, double* __restrict__ uv) {
+template <bool KEEP>
+__global__ void __launch_bounds__(512) k_driver_apply(const int64_t* __restrict__ tile_beg,
+                                                      const int32_t* __restrict__ tile_chart,
+                                                      const DriverState* __restrict__ st,
+                                                      const uint8_t* __restrict__ pinned,
+                                                      const double* __restrict__ pin_uv,
+                                                      const int64_t* __restrict__ row_of, DriverX X, int it, double* uv) {
   int64_t t = blockIdx.x;
   int c = tile_chart[t];
   int a = st[c].active;
-  if (a == 0) return;
+  if (a == 0 || (a == 2 && st[c].iters != it + 1)) return;
   double step = st[c].step;
-  for (int64_t v = tile_beg[2 * t] + threadIdx.x; v < tile_beg[2 * t + 1]; v += blockDim.x) {
-    double nu, nw;
-    new_uv_of(v, pinned, pin_uv, row_of, x, nu, nw);
-    double du = dsub(nu, uv[2 * v]), dw = dsub(nw, uv[2 * v + 1]);
-    uv[2 * v] = dadd(uv[2 * v], dmul(du, step));
-    uv[2 * v + 1] = dadd(uv[2 * v + 1], dmul(dw, step));
-  }
-}
-
-__global__ void k_driver_retire(DriverState* st, int64_t n_charts) {
-  int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < n_charts && st[c].active == 2) st[c].active = 0;
+  driver_verts<KEEP, 4>(tile_beg[2 * t], tile_beg[2 * t + 1], pinned, pin_uv, row_of, X, KEEP ? X.aux[c] : 0.0, uv,
+                        [&](int64_t v, double nu, double nw, double ou, double ow) {
+                          double du = dsub(nu, ou), dw = dsub(nw, ow);
+                          uv[2 * v] = dadd(ou, dmul(du, step));
+                          uv[2 * v + 1] = dadd(ow, dmul(dw, step));
+                        });
 }
 
 }  // namespace
@@ -665,15 +697,15 @@ namespace {
 using DriverHook = std::function<void(int, DriverState*, int*)>;
 }  // namespace
 
-static void driver_loop_dev(Ctx& ctx, DevBatch& bt, const DevSystem& sys, const double* x, int max_iter, double* uv,
+static void driver_loop_dev(Ctx& ctx, DevBatch& bt, const DriverX& X, int max_iter, double* uv,
                             std::vector<int32_t>& iters, std::vector<double>& err_accum, const DriverHook* hook);
 
 void driver_update(Ctx& ctx, DevBatch& bt, const DevSystem& sys, const double* x, int max_iter, double* uv,
                    std::vector<int32_t>& iters, std::vector<double>& err_accum) {
-  driver_loop_dev(ctx, bt, sys, x, max_iter, uv, iters, err_accum, nullptr);
+  driver_loop_dev(ctx, bt, DriverX{x, nullptr, nullptr}, max_iter, uv, iters, err_accum, nullptr);
 }
 
-static void driver_loop_dev(Ctx& ctx, DevBatch& bt, const DevSystem& sys, const double* x, int max_iter, double* uv,
+static void driver_loop_dev(Ctx& ctx, DevBatch& bt, const DriverX& X, int max_iter, double* uv,
                             std::vector<int32_t>& iters, std::vector<double>& err_accum, const DriverHook* hook) {
   cudaStream_t s = ctx.stream;
   Workspace& ws = ctx.ws;
@@ -711,8 +743,8 @@ static void driver_loop_dev(Ctx& ctx, DevBatch& bt, const DevSystem& sys, const 
   for (int it = 0; it < max_iter; ++it) {
     if (hook) (*hook)(it, st, n_active);
     if (NTL > 0) {
-      k_driver_partials<<<(unsigned)NTL, 256, 0, s>>>(d_tab, d_tchart, NTL, st, bt.pinned, bt.pin_uv, bt.row_of, x, uv,
-                                                      part);
+      auto k = hook ? k_driver_partials<true> : k_driver_partials<false>;
+      k<<<(unsigned)NTL, 256, 0, s>>>(d_tab, d_tchart, st, bt.pinned, bt.pin_uv, bt.row_of, X, uv, part);
       count_launches(1);
       RUV_LAUNCH_CHECK();
     }
@@ -720,13 +752,14 @@ static void driver_loop_dev(Ctx& ctx, DevBatch& bt, const DevSystem& sys, const 
     count_launches(1);
     RUV_LAUNCH_CHECK();
     if (NTL > 0) {
-      k_driver_apply<<<(unsigned)NTL, 256, 0, s>>>(d_tab, d_tchart, NTL, st, bt.pinned, bt.pin_uv, bt.row_of, x, uv);
+      auto k = hook ? k_driver_apply<true> : k_driver_apply<false>;
+      k<<<(unsigned)NTL, 512, 0, s>>>(d_tab, d_tchart, st, bt.pinned, bt.pin_uv, bt.row_of, X, it, uv);
       count_launches(1);
       RUV_LAUNCH_CHECK();
     }
-    k_driver_retire<<<div_up(NC, 256), 256, 0, s>>>(st, NC);
-    count_launches(1);
-    RUV_LAUNCH_CHECK();
+    // most loops end within two iterations; a long one asks only every eighth time (its kernels return
+    // at once for charts that have ended), so that the launches of an iteration run ahead
+    if (it >= 4 && it + 1 < max_iter && (it & 7) != 7) continue;
     RUV_CUDA(cudaMemcpyAsync(h_active, n_active, sizeof(int), cudaMemcpyDeviceToHost, s));
     RUV_CUDA(cudaStreamSynchronize(s));
     if (*h_active <= 0) break;
@@ -845,52 +878,78 @@ __global__ void k_km_u(const int64_t* __restrict__ tab, const int32_t* __restric
   }
 }
 
-// per triangle tile of an active chart: the sum of the area terms of uv
-__global__ void k_km_area(const int64_t* __restrict__ ttab, const int32_t* __restrict__ ttchart,
-                          const DriverState* __restrict__ st, const int32_t* __restrict__ tri_g,
-                          const double* __restrict__ uv, double* __restrict__ part) {
-  __shared__ double sh[32];
-  const int64_t tl = blockIdx.x;
-  if (!st[ttchart[tl]].active) return;
-  double acc[1] = {0.0};
-  for (int64_t t = ttab[2 * tl] + threadIdx.x; t < ttab[2 * tl + 1]; t += blockDim.x)
-    acc[0] += km_area_term(uv, tri_g[3 * t], tri_g[3 * t + 1], tri_g[3 * t + 2]);
-  block_sum<1>(acc, sh);
-  if (threadIdx.x == 0) part[tl] = acc[0];
+// every free vertex's triangles in record order, once for all iterations: entry rec_off[v] / 2 + k (two
+// records for each triangle) holds triangle k's vertices and which of them v is
+__global__ void k_km_entries(int64_t nv, const uint8_t* __restrict__ pinned, const int64_t* __restrict__ rec_off,
+                             const int2* __restrict__ rec, const int32_t* __restrict__ tri_g, int4* __restrict__ ent) {
+  const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= nv || pinned[v]) return;
+  int4* e = ent + rec_off[v] / 2;
+  km_vertex_tris(v, rec_off, rec, tri_g,
+                 [&](int64_t t, int m) { *e++ = make_int4(tri_g[3 * t], tri_g[3 * t + 1], tri_g[3 * t + 2], m); });
 }
 
-// per vertex tile of an active chart: the area gradient of every free vertex (lscm.rs:133-155,
-// its triangles in record order) dotted with y_b and y_u, and the count of its nonzero
-// components
-__global__ void k_km_grad(const int64_t* __restrict__ tab, const int32_t* __restrict__ tchart,
-                          const DriverState* __restrict__ st, const uint8_t* __restrict__ pinned,
-                          const int64_t* __restrict__ row_of, const int64_t* __restrict__ rec_off,
-                          const int2* __restrict__ rec, const int32_t* __restrict__ tri_g, const double* __restrict__ uv,
-                          const double* __restrict__ yb, const double* __restrict__ yu, double* __restrict__ part) {
+// The first ntt CTAs: per triangle tile of an active chart, the sum of the area terms of uv.  The
+// others: per vertex tile, the area gradient of every free vertex (lscm.rs:133-155, its triangles in
+// record order) dotted with y_b and y_u, and the count of its nonzero components.  A few hundred CTAs at
+// most on small charts, so a launch takes as long as a vertex's chain of loads: its entries come four
+// at a time (triangle by triangle through the records: 27.5 us for 32 charts of up to 3,000 vertices; with
+// this and the driver's batched loads, two launches less and a host check every eighth iteration, their
+// 100 iterations and solve take 19.5 ms against 23.0).
+__global__ void __launch_bounds__(256) k_km_partials(int64_t ntt, const int64_t* __restrict__ ttab,
+                                                     const int32_t* __restrict__ ttchart, const int64_t* __restrict__ vtab,
+                                                     const int32_t* __restrict__ vtchart, const DriverState* __restrict__ st,
+                                                     const uint8_t* __restrict__ pinned, const int64_t* __restrict__ row_of,
+                                                     const int64_t* __restrict__ rec_off, const int4* __restrict__ ent,
+                                                     const int32_t* __restrict__ tri_g, const double* __restrict__ uv,
+                                                     const double* __restrict__ yb, const double* __restrict__ yu,
+                                                     double* __restrict__ apart, double* __restrict__ gpart) {
   __shared__ double sh[96];
-  const int64_t tl = blockIdx.x;
-  if (!st[tchart[tl]].active) return;
+  if ((int64_t)blockIdx.x < ntt) {
+    const int64_t tl = blockIdx.x;
+    if (st[ttchart[tl]].active != 1) return;
+    double acc[1] = {0.0};
+    for (int64_t t = ttab[2 * tl] + threadIdx.x; t < ttab[2 * tl + 1]; t += blockDim.x)
+      acc[0] += km_area_term(uv, tri_g[3 * t], tri_g[3 * t + 1], tri_g[3 * t + 2]);
+    block_sum<1>(acc, sh);
+    if (threadIdx.x == 0) apart[tl] = acc[0];
+    return;
+  }
+  const int64_t tl = (int64_t)blockIdx.x - ntt;
+  if (st[vtchart[tl]].active != 1) return;
   double acc[3] = {0.0, 0.0, 0.0};
-  for (int64_t v = tab[2 * tl] + threadIdx.x; v < tab[2 * tl + 1]; v += blockDim.x) {
+  for (int64_t v = vtab[2 * tl] + threadIdx.x; v < vtab[2 * tl + 1]; v += blockDim.x) {
     if (pinned[v]) continue;
     double gu = 0.0, gv = 0.0;
-    km_vertex_tris(v, rec_off, rec, tri_g, [&](int64_t t, int m) {
-      const int32_t a = tri_g[3 * t], b = tri_g[3 * t + 1], c = tri_g[3 * t + 2];
-      const double x0 = uv[2 * a], y0 = uv[2 * a + 1], x1 = uv[2 * b], y1 = uv[2 * b + 1], x2 = uv[2 * c],
-                   y2 = uv[2 * c + 1];
-      const double sgd = dmul(0.5, dadd(dadd(dmul(x0, dsub(y2, y1)), dmul(x1, dsub(y0, y2))), dmul(x2, dsub(y1, y0))));
-      const double h = sgd > 0.0 ? 0.5 : -0.5;
-      if (m == 0) {
-        gu = dadd(gu, dmul(dsub(y2, y1), h));
-        gv = dadd(gv, dmul(dsub(x1, x2), h));
-      } else if (m == 1) {
-        gu = dadd(gu, dmul(dsub(y0, y2), h));
-        gv = dadd(gv, dmul(dsub(x2, x0), h));
-      } else {
-        gu = dadd(gu, dmul(dsub(y1, y0), h));
-        gv = dadd(gv, dmul(dsub(x0, x1), h));
+    const int64_t beg = rec_off[v] / 2, end = rec_off[v + 1] / 2;
+    constexpr int U = 4;
+    for (int64_t e = beg; e < end; e += U) {
+      int4 q[U];
+      double x[U][3], y[U][3];
+#pragma unroll
+      for (int k = 0; k < U; ++k) q[k] = ent[min(e + k, end - 1)];
+#pragma unroll
+      for (int k = 0; k < U; ++k) {
+        const int32_t id[3] = {q[k].x, q[k].y, q[k].z};
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          x[k][j] = uv[2 * (int64_t)id[j]];
+          y[k][j] = uv[2 * (int64_t)id[j] + 1];
+        }
       }
-    });
+#pragma unroll
+      for (int k = 0; k < U; ++k) {
+        if (e + k >= end) break;
+        const double x0 = x[k][0], y0 = y[k][0], x1 = x[k][1], y1 = y[k][1], x2 = x[k][2], y2 = y[k][2];
+        const double sgd = dmul(0.5, dadd(dadd(dmul(x0, dsub(y2, y1)), dmul(x1, dsub(y0, y2))), dmul(x2, dsub(y1, y0))));
+        const double h = sgd > 0.0 ? 0.5 : -0.5;
+        const int m = q[k].w;
+        const double du = m == 0 ? dsub(y2, y1) : m == 1 ? dsub(y0, y2) : dsub(y1, y0);
+        const double dv = m == 0 ? dsub(x1, x2) : m == 1 ? dsub(x2, x0) : dsub(x0, x1);
+        gu = dadd(gu, dmul(du, h));
+        gv = dadd(gv, dmul(dv, h));
+      }
+    }
     const int64_t r = row_of[v];
     acc[0] += gu * yb[2 * r] + gv * yb[2 * r + 1];
     acc[1] += gu * yu[2 * r] + gv * yu[2 * r + 1];
@@ -898,9 +957,9 @@ __global__ void k_km_grad(const int64_t* __restrict__ tab, const int32_t* __rest
   }
   block_sum<3>(acc, sh);
   if (threadIdx.x == 0) {
-    part[3 * tl] = acc[0];
-    part[3 * tl + 1] = acc[1];
-    part[3 * tl + 2] = acc[2];
+    gpart[3 * tl] = acc[0];
+    gpart[3 * tl + 1] = acc[1];
+    gpart[3 * tl + 2] = acc[2];
   }
 }
 
@@ -910,7 +969,7 @@ __global__ void k_km_aux(const int64_t* __restrict__ chart_ttile, const int64_t*
                          const double* __restrict__ target, int it, double* __restrict__ aux, int* __restrict__ n_active) {
   __shared__ double sh[128];
   const int64_t c = blockIdx.x;
-  if (!st[c].active) return;
+  if (st[c].active != 1) return;
   double acc[4] = {0.0, 0.0, 0.0, 0.0};
   for (int64_t t = chart_ttile[c] + threadIdx.x; t < chart_ttile[c + 1]; t += blockDim.x) acc[0] += apart[t];
   for (int64_t t = chart_vtile[c] + threadIdx.x; t < chart_vtile[c + 1]; t += blockDim.x) {
@@ -931,22 +990,6 @@ __global__ void k_km_aux(const int64_t* __restrict__ chart_ttile, const int64_t*
   aux[c] = a;
 }
 
-// x = y_b - aux y_u on the rows of active charts
-__global__ void k_km_x(const int64_t* __restrict__ tab, const int32_t* __restrict__ tchart,
-                       const DriverState* __restrict__ st, const uint8_t* __restrict__ pinned,
-                       const int64_t* __restrict__ row_of, const double* __restrict__ yb, const double* __restrict__ yu,
-                       const double* __restrict__ aux, double* __restrict__ x) {
-  const int64_t tl = blockIdx.x;
-  const int c = tchart[tl];
-  if (!st[c].active) return;
-  const double a = aux[c];
-  for (int64_t v = tab[2 * tl] + threadIdx.x; v < tab[2 * tl + 1]; v += blockDim.x) {
-    if (pinned[v]) continue;
-    const int64_t r = row_of[v];
-    x[2 * r] = yb[2 * r] - a * yu[2 * r];
-    x[2 * r + 1] = yb[2 * r + 1] - a * yu[2 * r + 1];
-  }
-}
 }  // namespace
 
 // The slack column u of the KeepMetric system (2 * n_rows, device) after assemble_lscm.
@@ -1030,18 +1073,20 @@ void driver_keep_metric(Ctx& ctx, DevBatch& bt, const DevSystem& sys, const doub
   double* apart = ws.get<double>("kmd.apart", std::max<int64_t>(NTT, 1));
   double* gpart = ws.get<double>("kmd.gpart", 3 * std::max<int64_t>(NTL, 1));
   double* aux = ws.get<double>("kmd.aux", std::max<int64_t>(NC, 1));
-  double* x = ws.get<double>("kmd.x", 2 * std::max<int64_t>(sys.n_rows, 1));
+  int4* ent = ws.get<int4>("kmd.ent", std::max<int64_t>(3 * bt.n_tris, 1));
+  if (bt.n_verts > 0) {
+    k_km_entries<<<div_up(bt.n_verts, 256), 256, 0, s>>>(bt.n_verts, bt.pinned, bt.rec_off, bt.rec, bt.tri_g, ent);
+    count_launches(1);
+  }
   DriverHook hook = [&](int it, DriverState* st, int* n_active) {
-    if (NTT > 0) k_km_area<<<(unsigned)NTT, 256, 0, s>>>(d_ttab, d_tch, st, bt.tri_g, uv, apart);
-    if (NTL > 0)
-      k_km_grad<<<(unsigned)NTL, 256, 0, s>>>(d_vtab, d_vch, st, bt.pinned, bt.row_of, bt.rec_off, bt.rec, bt.tri_g, uv,
-                                              yb, yu, gpart);
+    if (NTT + NTL > 0)
+      k_km_partials<<<(unsigned)(NTT + NTL), 256, 0, s>>>(NTT, d_ttab, d_tch, d_vtab, d_vch, st, bt.pinned, bt.row_of,
+                                                          bt.rec_off, ent, bt.tri_g, uv, yb, yu, apart, gpart);
     k_km_aux<<<(unsigned)NC, 128, 0, s>>>(d_tct, d_vct, st, apart, gpart, d_target, it, aux, n_active);
-    if (NTL > 0) k_km_x<<<(unsigned)NTL, 256, 0, s>>>(d_vtab, d_vch, st, bt.pinned, bt.row_of, yb, yu, aux, x);
-    count_launches(4);
+    count_launches(2);
     RUV_LAUNCH_CHECK();
   };
-  driver_loop_dev(ctx, bt, sys, x, max_iter, uv, iters, err_accum, &hook);
+  driver_loop_dev(ctx, bt, DriverX{yb, yu, aux}, max_iter, uv, iters, err_accum, &hook);
 }
 
 namespace {
