@@ -163,25 +163,7 @@ __device__ __forceinline__ int32_t narrow_row_base(int32_t cb, int64_t i) {
   return NW == 2 ? (int32_t)i - kRowRelBias : NW == 1 ? cb : 0;
 }
 
-template <int NV, class A>
-__device__ __forceinline__ void block_sum_t(A (&v)[NV], A* sh) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-  for (int k = 0; k < NV; ++k) v[k] = warp_sum(v[k]);
-  __syncthreads();
-  if (lane == 0)
-#pragma unroll
-    for (int k = 0; k < NV; ++k) sh[k * 32 + wid] = v[k];
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < NV; ++k) {
-    A t = lane < nw ? sh[k * 32 + lane] : A(0);
-    v[k] = warp_sum(t);
-  }
-  __syncthreads();
-}
-
-// The same totals in thread 0 alone, for one use of `sh` in a kernel: the last step runs in one warp (in
+// The totals of block_sum in thread 0 alone, for one use of `sh` in a kernel: the last step runs in one warp (in
 // FP64 every warp that repeats it costs the SM's FP64 pipe 100 clocks a value).
 template <int NV, class A>
 __device__ __forceinline__ void block_sum_first(A (&v)[NV], A* sh) {

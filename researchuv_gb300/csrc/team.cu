@@ -11,8 +11,8 @@
 // step, where the lockstep loop streams the whole batch from HBM in every kernel.
 //
 // A team is 1 to 16 CTAs of 512 threads (one row per thread where the chart is small enough); the
-// rule is in team_size.  Rows go round-robin over the team in blocks of 512, so consecutive threads
-// read consecutive rows.  Vectors live in global memory (they are the launch loop's own arrays) and
+// rule is in team_solve), each with a contiguous share of the chart's rows, consecutive rows on
+// consecutive threads.  Vectors live in global memory (they are the launch loop's own arrays) and
 // are L1- or L2-resident; the cluster barrier's release/acquire orders them.  Scalars are formed by
 // one lane per CTA from the same partial sums in the same order, so every CTA of a team decides
 // alike and results do not depend on timing.  (FP64 adds have 64 clocks of latency and 1.6 results

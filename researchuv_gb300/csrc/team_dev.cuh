@@ -156,12 +156,5 @@ __device__ __forceinline__ V<S, NR> entries_dot(int32_t lo, int32_t hi, Val val,
   }
   return s;
 }
-template <class S, int NR, class Get>
-__device__ __forceinline__ V<S, NR> row_dot(const int32_t* rp, const Cols& cols, const S* vals, int32_t i, Get get) {
-  const int32_t rb = cols.base(i);
-  return entries_dot<S, NR>(
-      __ldg(rp + i), __ldg(rp + i + 1), [&](int32_t e) { return __ldg(vals + e); },
-      [&](int32_t e) { return cols.at(e, rb); }, get);
-}
 
 }  // namespace ruv
