@@ -74,3 +74,16 @@ def test_dense_block_solves_alone(n):
     assert got is not None, s.last_error
     x = np.linalg.solve(m.toarray(), b)
     assert np.abs(np.asarray(got[0]) - x).max() <= 1e-10 * np.abs(x).max()
+
+
+# the scan's one block, its blocks that add their totals themselves (to 1024 blocks of n + 1 values), the next
+@pytest.mark.parametrize("n", [1022, 1023, 1024, 2048, 1024 * 1024 - 1, 1024 * 1024])
+def test_scan_edges_number_the_aggregates(n):
+    m = sp.diags([-np.ones(n - 1), 2.5 * np.ones(n), -np.ones(n - 1)], [-1, 0, 1]).tocsr()
+    L = R.GpuSolver(R.Context(0)).amg_level(_csr(m), 0, True)
+    agg, nc = L["agg"], L["next_rows"]
+    assert L["rows"] == n and 0 < nc < n
+    assert agg.min() == 0 and agg.max() == nc - 1
+    assert np.bincount(agg, minlength=nc).min() >= 1
+    ptr = np.asarray(L["P"][0])
+    assert ptr[0] == 0 and ptr[-1] == len(L["P"][1]) and np.diff(ptr).min() >= 1
