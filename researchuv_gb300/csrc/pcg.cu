@@ -1663,6 +1663,8 @@ std::vector<ChartResult> pcg_solve(Ctx& ctx, DevSystem& sys, double* x, const So
   std::vector<ChartResult> res(NC);
   for (int64_t c = 0; c < NC; ++c) {
     const ChartState& cs = out[c];
+    if (cs.status == RUV_ERR_TIMEOUT)
+      throw Error{RUV_ERR_TIMEOUT, "team solver: a bounded wait for a team's sums ran out (RUV_SPIN_LIMIT)"};
     res[c].status = cs.status;
     res[c].iters = cs.iters;
     res[c].refinements = cs.refinements;

@@ -40,6 +40,7 @@ struct TeamShared {
   double due, due2;  // the residual norm at which something is due, and its square_of
   float due2f;
   int flag;
+  uint64_t left[kTeamMaxCtas];  // per CTA of the team: kStaying, or the barrier it left before and how (team_leave)
   int32_t lvl_row[kTeamMaxLevels];  // the chart's first row and row count per level
   int32_t lvl_n[kTeamMaxLevels];
 };
@@ -70,16 +71,25 @@ __device__ __forceinline__ void st_async(const unsigned long long* p, const uint
                : "memory");
 }
 
+// v into CTA `rank`'s copy of *p
+__device__ __forceinline__ void st_cluster(const uint64_t* p, uint32_t rank, uint64_t v) {
+  uint32_t d;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(smem_addr(p)), "r"(rank));
+  asm volatile("st.shared::cluster.b64 [%0], %1;" ::"r"(d), "l"(v) : "memory");
+}
+
 struct Team {
   int ctas, rank, threads, id;  // id: this thread's number in the team
   int buf;
   uint32_t phase[2];
+  mutable uint32_t bars;  // cluster barriers passed: the same number in every CTA at the same barrier
   // every thread of the team; global and shared writes before it are visible after it
   __device__ __forceinline__ void bar() const {
     if (ctas == 1) {
       __syncthreads();
     } else {
       asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
+      ++bars;
     }
   }
   // the same where a one-CTA team is already past a block barrier (team_reduce)
@@ -89,19 +99,49 @@ struct Team {
 };
 
 // tries of the wait for a team's partial sums (each of them suspends for a while by itself): a few
-// seconds, far above the longest step
+// seconds, far above the longest step (RUV_SPIN_LIMIT overrides; 0: every wait runs out at once)
 constexpr int64_t kTeamSpin = int64_t(1) << 22;
 
 enum : int { kGo = 0, kRefresh = 1, kStop = 2, kLost = 3 };
 
+// The end of a team's kernel, for every CTA and however it got here; whether any wait of the team ran
+// out.  A CTA whose wait for the others' sums ran out cannot know which way they go on, so it comes
+// here while they may still be on their way -- and they need it: a cluster barrier counts every
+// CTA, and shared memory that a peer may still write has to stay.  So it meets their barriers from here,
+// one after another wherever theirs are in the code, until all have come: it sends no more sums, so the
+// wait of each peer's next reduction runs out too, or that peer has ended with this one's last sums.
+// A CTA announces itself, before its next barrier, by that barrier's number, and an announcement
+// counts from that barrier on: an early look at a later one would send one CTA out ahead of the others.
+constexpr uint32_t kStaying = 0, kLeft = 1, kLeftLost = 2;
+__device__ __forceinline__ bool team_leave(const Team& tm, TeamShared& sh, bool lost) {
+  if (tm.ctas == 1) return false;
+  if ((int)threadIdx.x < tm.ctas)
+    st_cluster(&sh.left[tm.rank], threadIdx.x, ((uint64_t)(tm.bars + 1) << 32) | (lost ? kLeftLost : kLeft));
+  bool all, any;
+  do {
+    tm.bar();
+    all = true;
+    any = false;
+    for (int k = 0; k < tm.ctas; ++k) {
+      const uint64_t u = *const_cast<volatile uint64_t*>(&sh.left[k]);
+      all = all && (uint32_t)u != kStaying && (int32_t)(tm.bars - (uint32_t)(u >> 32)) >= 0;
+      any = any || (uint32_t)u == kLeftLost;
+    }
+  } while (!all);
+  if (any)  // asynchronous stores of sums that nobody waited for land within a microsecond or so
+    for (const long long t0 = clock64(); clock64() - t0 < (1 << 18);) {
+    }
+  return any;
+}
+
 // Sum of every thread's v over the team in a fixed order, then fn(totals) in one lane of every CTA;
-// its return value comes back to every thread.  The CTAs' sums travel as asynchronous stores into
+// its return value comes back to every thread (kLost: the wait for the sums ran out).  The CTAs' sums travel as asynchronous stores into
 // each peer's shared memory, counted by an mbarrier there, so nothing waits for global stores in
 // flight: a cluster barrier took 1,470 clocks behind a step's stores where it takes 600 alone.  No
 // thread gets past this before every thread of the team has reached it; it publishes no global
 // memory in a team of several CTAs (Team::publish does).
 template <int NV, class T, class Fn>
-__device__ __forceinline__ int team_reduce(Team& tm, TeamShared& sh, const T (&v)[NV], Fn fn) {
+__device__ __forceinline__ int team_reduce(Team& tm, TeamShared& sh, int64_t limit, const T (&v)[NV], Fn fn) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, buf = tm.buf;
   T* part = reinterpret_cast<T*>(sh.part[buf]);
   T w[NV];
@@ -131,7 +171,7 @@ __device__ __forceinline__ int team_reduce(Team& tm, TeamShared& sh, const T (&v
       if (lane < tm.ctas)
 #pragma unroll
         for (int k = 0; k < NV; ++k) st_async(&sh.slot[buf][k][tm.rank], &sh.slot_bar[buf], lane, sc_bits(tot[k]));
-      ok = mbar_wait(&sh.slot_bar[buf], tm.phase[buf], kTeamSpin);
+      ok = mbar_wait(&sh.slot_bar[buf], tm.phase[buf], limit);
       ok = __all_sync(0xffffffffu, ok);
 #pragma unroll
       for (int k = 0; k < NV; ++k) {
@@ -510,12 +550,14 @@ __global__ void __launch_bounds__(kTeamThreads, team_per_sm<S, PCK>())
   tm.id = tm.rank * kTeamThreads + (int)threadIdx.x;
   tm.buf = 0;
   tm.phase[0] = tm.phase[1] = 0;
+  tm.bars = 0;
   const int chart = A.order[cluster_id()];
   auto set_due = [&](double norm) {
     sh.due = fmax(norm, sh.st.tol_abs);
     if constexpr (mixed) sh.due2f = square_of(0.0f, sh.due);
     else sh.due2 = square_of(0.0, sh.due);
   };
+  if (threadIdx.x < kTeamMaxCtas) sh.left[threadIdx.x] = kStaying;
   if (threadIdx.x == 0) {
     sh.st = P.st[chart];
     set_due(mixed ? P.delta * sh.st.r_ref : 0.0);
@@ -622,7 +664,7 @@ __global__ void __launch_bounds__(kTeamThreads, team_per_sm<S, PCK>())
           });
       for (int32_t i = R0 + (int32_t)threadIdx.x; i < R1; i += kTeamThreads) dots(i, ldv<S, NR>(P.z, i));
     }
-    const int flag = team_reduce<2, S>(tm, sh, acc, fn);
+    const int flag = team_reduce<2, S>(tm, sh, P.spin_limit, acc, fn);
     if (PCK == 1) tm.publish();  // z (the sweeps' last barrier has published theirs)
     return flag;
   };
@@ -665,7 +707,7 @@ __global__ void __launch_bounds__(kTeamThreads, team_per_sm<S, PCK>())
 #pragma unroll
       for (int c = 0; c < NR; ++c) pq[0] += pi.c[c] * s.c[c];
     }
-    flag = team_reduce<1, S>(tm, sh, pq, [&](const Sc (&t)[1]) {
+    flag = team_reduce<1, S>(tm, sh, P.spin_limit, pq, [&](const Sc (&t)[1]) {
       if (vanishes(t[0]) || !isfinite(sc_hi(t[0]))) {  // solver.rs:505-508
         sh.st.status = RUV_ERR_BREAKDOWN;
         return (int)kStop;
@@ -701,7 +743,7 @@ __global__ void __launch_bounds__(kTeamThreads, team_per_sm<S, PCK>())
       else sh.beta = beta;
       sh.s_rz = sc_bits(rznew);
     };
-    flag = team_reduce<2, S>(tm, sh, rr, [&](const Sc (&t)[2]) {
+    flag = team_reduce<2, S>(tm, sh, P.spin_limit, rr, [&](const Sc (&t)[2]) {
       sh.st.iters += 1;
       bool due;
       if constexpr (mixed) due = at_most(t[0].h, sh.due, sh.due2f);
@@ -802,7 +844,7 @@ __global__ void __launch_bounds__(kTeamThreads, team_per_sm<S, PCK>())
           stv<float, NR>(P.r, i, rv);
           put_r(i, rv);
         }
-        flag = team_reduce<2, float>(tm, sh, acc, [&](const Pair (&t)[2]) {
+        flag = team_reduce<2, float>(tm, sh, P.spin_limit, acc, [&](const Pair (&t)[2]) {
           const double inv = 1.0 / ((double)rsc * (double)rsc);
           sh.st.refinements += 1;
           sh.st.rr = t[0].f64() * inv;
@@ -874,14 +916,14 @@ __global__ void __launch_bounds__(kTeamThreads, team_per_sm<S, PCK>())
       stv<double, NR>(P.x64, i, x);
     }
   }
+  const bool lost = team_leave(tm, sh, flag == kLost);
   if (tm.id == 0) {
-    if (flag == kLost) sh.st.status = RUV_ERR_TIMEOUT;
+    if (lost) sh.st.status = RUV_ERR_TIMEOUT;
     sh.st.state = kDone;
     sh.st.refresh = 0;
     P.st[chart] = sh.st;
     atomicSub(P.n_active, 1);
   }
-  if (tm.ctas > 1) tm.bar();  // no CTA leaves while a peer may still write its shared memory
 }
 
 // ---------------------------------------------------------------- which charts, and how many CTAs
@@ -943,13 +985,15 @@ void Ctx::team_streams(int n) {
 }
 
 template <class S, int NR>
-int64_t team_solve(Ctx& ctx, const DevSystem& sys, const TeamLoop<S>& loop, const TeamPrecond* pc) {
+int64_t team_solve(Ctx& ctx, const DevSystem& sys, TeamLoop<S> loop, const TeamPrecond* pc) {
   const int64_t NC = sys.n_charts;
   const int kind = pc ? pc->kind : 0;
   constexpr bool mixed = std::is_same<S, float>::value;
   auto rows_of = [&](int64_t c) { return sys.h_chart_row[c + 1] - sys.h_chart_row[c]; };
   int64_t left = 0, largest = 0;
   for (int64_t c = 0; c < NC; ++c) largest = std::max(largest, rows_of(c));
+  const char* le = std::getenv("RUV_SPIN_LIMIT");
+  loop.spin_limit = le ? std::max<int64_t>(0, std::atoll(le)) : kTeamSpin;
   const char* re = std::getenv("RUV_TEAM_ROWS");
   // The largest chart a team of 16 SMs takes, where both ways were measured (ms, team / launch loop):
   // mixed Jacobi 39,000 rows 21.8 / 31.9, 89,000 57 / 60, 128,000 121 / 102; FP64 Jacobi, two columns,
@@ -1044,8 +1088,8 @@ int64_t team_solve(Ctx& ctx, const DevSystem& sys, const TeamLoop<S>& loop, cons
   return left;
 }
 
-template int64_t team_solve<float, 2>(Ctx&, const DevSystem&, const TeamLoop<float>&, const TeamPrecond*);
-template int64_t team_solve<double, 2>(Ctx&, const DevSystem&, const TeamLoop<double>&, const TeamPrecond*);
-template int64_t team_solve<double, 1>(Ctx&, const DevSystem&, const TeamLoop<double>&, const TeamPrecond*);
+template int64_t team_solve<float, 2>(Ctx&, const DevSystem&, TeamLoop<float>, const TeamPrecond*);
+template int64_t team_solve<double, 2>(Ctx&, const DevSystem&, TeamLoop<double>, const TeamPrecond*);
+template int64_t team_solve<double, 1>(Ctx&, const DevSystem&, TeamLoop<double>, const TeamPrecond*);
 
 }  // namespace ruv

@@ -68,15 +68,16 @@ struct TeamLoop {
   int64_t max_iter;
   double delta;
   int jacobi;  // plain loop: 1 Jacobi, 0 none
+  int64_t spin_limit = 0;  // tries of a wait for the team's sums (set by team_solve)
 };
 
 // Whether the kernels below may be used: not under RUV_TEAM=0 or a knob that picks a kernel of the
 // launch-per-step loop (RUV_LPR, RUV_SPMV_TMA, RUV_AMG_STAGE).
 bool teams_on(const Ctx& ctx);
 
-// Solves every chart that a team is the faster way for and marks it done in loop.st; returns the
-// number of charts left.
+// Solves every chart that a team is the faster way for and marks it done in loop.st (status
+// RUV_ERR_TIMEOUT where a bounded wait ran out); returns the number of charts left.
 template <class S, int NR>
-int64_t team_solve(Ctx& ctx, const DevSystem& sys, const TeamLoop<S>& loop, const TeamPrecond* pc);
+int64_t team_solve(Ctx& ctx, const DevSystem& sys, TeamLoop<S> loop, const TeamPrecond* pc);
 
 }  // namespace ruv
