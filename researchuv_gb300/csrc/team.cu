@@ -16,7 +16,8 @@
 // are L1- or L2-resident; the cluster barrier's release/acquire orders them.  Scalars are formed by
 // one lane per CTA from the same partial sums in the same order, so every CTA of a team decides
 // alike and results do not depend on timing.  (FP64 adds have 64 clocks of latency and 1.6 results
-// per clock and SM here: a reduction's last steps and the scalar divisions stay in one warp.)
+// per clock and SM here: a reduction's last steps and the scalar divisions stay in one warp, and the
+// divisions go to the integer pipe, fp64rn.cuh.)
 #include "team_dev.cuh"
 
 #include <algorithm>
@@ -30,15 +31,12 @@ constexpr int kTeamWarps = kTeamThreads / 32;
 constexpr int kTeamMaxCtas = 16;
 struct TeamShared {
   ChartState st;                    // lane 0's scalars (the same bits in every CTA of the team)
-  double part[2][2][kTeamWarps];    // [buffer][value][warp], as S
-  unsigned long long slot[2][2][kTeamMaxCtas];  // [buffer][value][CTA of the team]: a double or a Pair
+  double part[2][2][kTeamWarps];    // [buffer][value][warp]
+  double slot[2][2][kTeamMaxCtas];  // [buffer][value][CTA of the team]
   uint64_t slot_bar[2];             // completes when a buffer's slots have arrived
-  // the scalars, as a double or (mixed loop) a Pair, and what the vectors take of them
-  unsigned long long s_rz, s_alpha;
-  double alpha, beta;
-  float alpha32, beta32;
-  double due, due2;  // the residual norm at which something is due, and its square_of
-  float due2f;
+  double rz, alpha, beta;
+  float alpha32, beta32;  // what FP32 vectors take of them
+  double due, due2;       // the residual norm at which something is due, and its square_of
   int flag;
   uint64_t left[kTeamMaxCtas];  // per CTA of the team: kStaying, or the barrier it left before and how (team_leave)
   int32_t lvl_row[kTeamMaxLevels];  // the chart's first row and row count per level
@@ -61,13 +59,12 @@ __device__ __forceinline__ uint32_t cluster_id() {
   return r;
 }
 // v into CTA `rank`'s copy of *p, counted on its copy of *bar when it arrives
-__device__ __forceinline__ void st_async(const unsigned long long* p, const uint64_t* bar, uint32_t rank,
-                                         unsigned long long v) {
+__device__ __forceinline__ void st_async(const double* p, const uint64_t* bar, uint32_t rank, double v) {
   uint32_t d, m;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(smem_addr(p)), "r"(rank));
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(m) : "r"(smem_addr(bar)), "r"(rank));
   asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(d),
-               "l"(v), "r"(m)
+               "l"(__double_as_longlong(v)), "r"(m)
                : "memory");
 }
 
@@ -134,7 +131,8 @@ __device__ __forceinline__ bool team_leave(const Team& tm, TeamShared& sh, bool 
   return any;
 }
 
-// Sum of every thread's v over the team in a fixed order, then fn(totals) in one lane of every CTA;
+// Sum of every thread's v over the team in a fixed order -- in T within a warp (of FP32 rows at most 32 a
+// thread's share, below the launch loop's tile of 1,024), in FP64 from there -- then fn(totals) in one lane of every CTA;
 // its return value comes back to every thread (kLost: the wait for the sums ran out).  The CTAs' sums travel as asynchronous stores into
 // each peer's shared memory, counted by an mbarrier there, so nothing waits for global stores in
 // flight: a cluster barrier took 1,470 clocks behind a step's stores where it takes 600 alone.  No
@@ -143,43 +141,35 @@ __device__ __forceinline__ bool team_leave(const Team& tm, TeamShared& sh, bool 
 template <int NV, class T, class Fn>
 __device__ __forceinline__ int team_reduce(Team& tm, TeamShared& sh, int64_t limit, const T (&v)[NV], Fn fn) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, buf = tm.buf;
-  T* part = reinterpret_cast<T*>(sh.part[buf]);
-  T w[NV];
 #pragma unroll
-  for (int k = 0; k < NV; ++k) w[k] = warp_sum(v[k]);
-  if (lane == 0)
-#pragma unroll
-    for (int k = 0; k < NV; ++k) part[k * kTeamWarps + wid] = w[k];
+  for (int k = 0; k < NV; ++k) {
+    const T w = warp_sum(v[k]);
+    if (lane == 0) sh.part[buf][k][wid] = (double)w;
+  }
   __syncthreads();
-  using Sc = typename ScalarOf<T>::type;
   if (wid == 0) {
-    Sc tot[NV];
+    // each value in a half of the warp: one chain of FP64 additions for both
+    static_assert(NV <= 2 && kTeamWarps == 16 && kTeamMaxCtas == 16, "a value's terms are half a warp's lanes");
+    const int value = NV == 2 ? lane >> 4 : 0, term = lane & 15;
     bool ok = true;
+    double t = sh.part[buf][value][term];
 #pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      T t = part[k * kTeamWarps + (lane & (kTeamWarps - 1))];
-#pragma unroll
-      for (int o = kTeamWarps / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      if constexpr (sizeof(T) == 4) tot[k] = pair_of(t);
-      else tot[k] = t;
-    }
+    for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     if (tm.ctas > 1) {
       if (lane == 0)
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&sh.slot_bar[buf])),
                      "r"((uint32_t)(8 * NV * tm.ctas))
                      : "memory");
-      if (lane < tm.ctas)
-#pragma unroll
-        for (int k = 0; k < NV; ++k) st_async(&sh.slot[buf][k][tm.rank], &sh.slot_bar[buf], lane, sc_bits(tot[k]));
+      if (term < tm.ctas && lane < 16 * NV)
+        st_async(&sh.slot[buf][value][tm.rank], &sh.slot_bar[buf], term, t);
       ok = mbar_wait(&sh.slot_bar[buf], tm.phase[buf], limit);
       ok = __all_sync(0xffffffffu, ok);
-#pragma unroll
-      for (int k = 0; k < NV; ++k) {
-        Sc t = lane < tm.ctas ? sc_of_bits(Sc{}, sh.slot[buf][k][lane]) : sc_zero(Sc{});
-        for (int o = tm.ctas >> 1; o > 0; o >>= 1) t = sc_add(t, sc_shfl(t, o));
-        tot[k] = t;
-      }
+      t = term < tm.ctas ? sh.slot[buf][value][term] : 0.0;
+      for (int o = tm.ctas >> 1; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     }
+    double tot[NV];
+    tot[0] = t;
+    if constexpr (NV == 2) tot[1] = __shfl_sync(0xffffffffu, t, 16);
     if (lane == 0) sh.flag = ok ? fn(tot) : (int)kLost;
   }
   __syncthreads();
@@ -541,7 +531,6 @@ __global__ void __launch_bounds__(kTeamThreads, team_per_sm<S, PCK>())
            const __grid_constant__ TeamAmg M, const __grid_constant__ TeamIc0 I) {
   constexpr bool mixed = std::is_same<S, float>::value;
   using Vs = V<S, NR>;
-  using Sc = typename ScalarOf<S>::type;
   __shared__ TeamShared sh;
   Team tm;
   tm.ctas = (int)cluster_size();
@@ -554,14 +543,13 @@ __global__ void __launch_bounds__(kTeamThreads, team_per_sm<S, PCK>())
   const int chart = A.order[cluster_id()];
   auto set_due = [&](double norm) {
     sh.due = fmax(norm, sh.st.tol_abs);
-    if constexpr (mixed) sh.due2f = square_of(0.0f, sh.due);
-    else sh.due2 = square_of(0.0, sh.due);
+    sh.due2 = square_of(sh.due);
   };
   if (threadIdx.x < kTeamMaxCtas) sh.left[threadIdx.x] = kStaying;
   if (threadIdx.x == 0) {
     sh.st = P.st[chart];
     set_due(mixed ? P.delta * sh.st.r_ref : 0.0);
-    sh.s_rz = sc_bits(sc_from(Sc{}, sh.st.rz));
+    sh.rz = sh.st.rz;
     for (int k = 0; k < 2; ++k)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&sh.slot_bar[k])) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -690,8 +678,8 @@ __global__ void __launch_bounds__(kTeamThreads, team_per_sm<S, PCK>())
     if constexpr (PCK == 1)
       for (int32_t i = R0 + (int32_t)threadIdx.x; i < R1; i += kTeamThreads) put_r(i, ldv<S, NR>(P.r, i));
     tm.bar();
-    flag = apply([&](const Sc (&t)[2]) {
-      sh.s_rz = sc_bits(t[0]);
+    flag = apply([&](const double (&t)[2]) {
+      sh.rz = t[0];
       return (int)kGo;
     });
     for (int32_t i = R0 + (int32_t)threadIdx.x; i < R1; i += kTeamThreads) stv<S, NR>(P.p, i, zrow(i));
@@ -707,15 +695,13 @@ __global__ void __launch_bounds__(kTeamThreads, team_per_sm<S, PCK>())
 #pragma unroll
       for (int c = 0; c < NR; ++c) pq[0] += pi.c[c] * s.c[c];
     }
-    flag = team_reduce<1, S>(tm, sh, P.spin_limit, pq, [&](const Sc (&t)[1]) {
-      if (vanishes(t[0]) || !isfinite(sc_hi(t[0]))) {  // solver.rs:505-508
+    flag = team_reduce<1, S>(tm, sh, P.spin_limit, pq, [&](const double (&t)[1]) {
+      if (fabs(t[0]) <= 1e-300 || !isfinite(t[0])) {  // solver.rs:505-508
         sh.st.status = RUV_ERR_BREAKDOWN;
         return (int)kStop;
       }
-      const Sc alpha = sc_div(sc_of_bits(Sc{}, sh.s_rz), t[0]);
-      sh.s_alpha = sc_bits(alpha);
-      if constexpr (mixed) sh.alpha32 = alpha.h;
-      else sh.alpha = alpha;
+      sh.alpha = div_rn(sh.rz, t[0]);
+      sh.alpha32 = (float)sh.alpha;
       return (int)kGo;
     });
     if (flag >= kStop) break;
@@ -737,27 +723,24 @@ __global__ void __launch_bounds__(kTeamThreads, team_per_sm<S, PCK>())
       stv<S, NR>(P.r, i, rv);
       put_r(i, rv);
     }
-    auto new_beta = [&](Sc rznew) {
-      const Sc beta = sc_div(rznew, sc_of_bits(Sc{}, sh.s_rz));
-      if constexpr (mixed) sh.beta32 = beta.h;
-      else sh.beta = beta;
-      sh.s_rz = sc_bits(rznew);
+    auto new_beta = [&](double rznew) {
+      sh.beta = div_rn(rznew, sh.rz);
+      sh.beta32 = (float)sh.beta;
+      sh.rz = rznew;
     };
-    flag = team_reduce<2, S>(tm, sh, P.spin_limit, rr, [&](const Sc (&t)[2]) {
+    flag = team_reduce<2, S>(tm, sh, P.spin_limit, rr, [&](const double (&t)[2]) {
       sh.st.iters += 1;
-      bool due;
-      if constexpr (mixed) due = at_most(t[0].h, sh.due, sh.due2f);
-      else due = at_most(t[0], sh.due, sh.due2);
+      const bool due = at_most(t[0], sh.due, sh.due2);
       if constexpr (mixed) {
         // the FP32 residual only schedules true-residual refreshes
-        if (due || !isfinite(sc_hi(t[0])) || sh.st.iters >= P.max_iter) return (int)kRefresh;
+        if (due || !isfinite(t[0]) || sh.st.iters >= P.max_iter) return (int)kRefresh;
       } else {
-        sh.st.rr = sc_f64(t[0]);
+        sh.st.rr = t[0];
         if (due) {
           sh.st.status = RUV_OK;
           return (int)kStop;
         }
-        if (PCK != 0 && !isfinite(sc_hi(t[0]))) {
+        if (PCK != 0 && !isfinite(t[0])) {
           sh.st.status = RUV_ERR_BREAKDOWN;
           return (int)kStop;
         }
@@ -844,10 +827,10 @@ __global__ void __launch_bounds__(kTeamThreads, team_per_sm<S, PCK>())
           stv<float, NR>(P.r, i, rv);
           put_r(i, rv);
         }
-        flag = team_reduce<2, float>(tm, sh, P.spin_limit, acc, [&](const Pair (&t)[2]) {
+        flag = team_reduce<2, float>(tm, sh, P.spin_limit, acc, [&](const double (&t)[2]) {
           const double inv = 1.0 / ((double)rsc * (double)rsc);
           sh.st.refinements += 1;
-          sh.st.rr = t[0].f64() * inv;
+          sh.st.rr = t[0] * inv;
           const double rn = sqrt(sh.st.rr);
           if (rn <= sh.st.tol_abs) {
             sh.st.status = RUV_OK;
@@ -863,7 +846,7 @@ __global__ void __launch_bounds__(kTeamThreads, team_per_sm<S, PCK>())
           }
           sh.st.r_ref = rn;
           set_due(P.delta * rn);
-          if constexpr (PCK == 0 && mixed) new_beta(pair_of((P.jacobi ? t[1] : t[0]).f64() * inv));
+          if constexpr (PCK == 0 && mixed) new_beta((P.jacobi ? t[1] : t[0]) * inv);
           return (int)kGo;
         });
         if (flag >= kStop) break;
@@ -871,15 +854,14 @@ __global__ void __launch_bounds__(kTeamThreads, team_per_sm<S, PCK>())
     }
     if constexpr (PCK != 0) {
       tm.publish();  // r, for the rows other CTAs own
-      flag = apply([&](const Sc (&t)[2]) {
+      flag = apply([&](const double (&t)[2]) {
         // flexible (Polak-Ribiere) for the V-cycle using r_new - r_old = -alpha q, Fletcher-Reeves
         // for IC(0) and right after a refresh (pcg.cu k_chart_beta_pc)
-        Sc beta = sc_div(PCK == 1 && !fresh ? sc_neg_mul(sc_of_bits(Sc{}, sh.s_alpha), t[1]) : t[0],
-                         sc_of_bits(Sc{}, sh.s_rz));
-        if (!isfinite(sc_hi(beta))) beta = sc_zero(beta);
-        if constexpr (mixed) sh.beta32 = beta.h;
-        else sh.beta = beta;
-        sh.s_rz = sc_bits(t[0]);
+        double beta = div_rn(PCK == 1 && !fresh ? -sh.alpha * t[1] : t[0], sh.rz);
+        if (!isfinite(beta)) beta = 0.0;
+        sh.beta = beta;
+        sh.beta32 = (float)beta;
+        sh.rz = t[0];
         return (int)kGo;
       });
       if (flag >= kStop) break;
