@@ -266,10 +266,11 @@ ruv_status ruv_rectangularize(ruv_ctx* ctx, const double* uv, const uint8_t* bor
 ruv_status ruv_host_alloc(ruv_ctx* ctx, int64_t bytes, void** out);
 void ruv_host_free(void* p);
 
-/* Self-test of the assembly's FP64 division and square root (computed on the integer and
- * FP32 pipes, bit-identical to the IEEE operations by design): n seeded inputs of class
- * `mode` (0-2: quotients -- moderate exponents, arbitrary bit patterns, near midpoints;
- * 3-5: square roots -- moderate exponents, arbitrary bit patterns, near perfect squares)
+/* Self-test of the library's FP64 division and square root (computed on the integer and
+ * FP32 pipes, bit-identical to the IEEE operations by design) and of its division by a kept
+ * reciprocal: n seeded inputs of class `mode` (0-2: quotients -- moderate exponents, arbitrary bit
+ * patterns, near midpoints; 3-5: square roots -- moderate exponents, arbitrary bit patterns, near
+ * perfect squares; 6-8: quotients by the reciprocal, the classes of 0-2, 7 with its cut-offs)
  * compared bit for bit with the hardware operations.  *mismatches = the count; first4 =
  * (a, b, got, want) of the first mismatch.  No reference counterpart: a diagnostic. */
 ruv_status ruv_selftest_fp64(ruv_ctx* ctx, int mode, uint64_t seed, int64_t n, int64_t* mismatches, double* first4);

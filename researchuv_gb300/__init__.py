@@ -669,7 +669,8 @@ def rectangularize(ctx: Context, uv, border, n_charts: int):
 
 def selftest_fp64(ctx: Context, mode: int, seed: int, n: int):
     """Bitwise comparison of the assembly's FP64 division / square root (integer and FP32
-    pipes) with the hardware operations on n seeded inputs of class `mode` (0-5).  Returns
+    pipes; modes 0-5) or of the division by a kept reciprocal (6-8) with the hardware
+    operations on n seeded inputs of class `mode`.  Returns
     (mismatches, (a, b, got, want) of the first)."""
     bad = _i64(0)
     first = np.zeros(4, np.float64)

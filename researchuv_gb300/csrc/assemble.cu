@@ -1097,7 +1097,8 @@ namespace {
 //    quotients leaving the normal range); 2: quotients near a midpoint (a = b q rounded, moved
 //    by -2..2 ulps); 3: square roots, exponents within +-60; 4: square roots of arbitrary bit
 //    patterns; 5: square roots near perfect squares (s^2 exact for s < 2^26, moved by -2..2
-//    ulps, scaled by 4^k).
+//    ulps, scaled by 4^k); 6: div_by on the classes of 0, 7: on those of 1, exponents at its cut-offs
+//    and zeros over every divisor; 8: on those of 2.
 __device__ __forceinline__ uint64_t splitmix64(uint64_t z) {
   z += 0x9E3779B97F4A7C15ull;
   z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
@@ -1115,11 +1116,24 @@ __global__ void k_fp64_selftest(int mode, uint64_t seed, int64_t n, unsigned lon
   const uint64_t r0 = splitmix64(seed + 3 * (uint64_t)i), r1 = splitmix64(seed + 3 * (uint64_t)i + 1),
                  r2 = splitmix64(seed + 3 * (uint64_t)i + 2);
   double a = 0.0, b = 0.0, got, want;
-  if (mode <= 2) {
-    if (mode == 0) {
+  if (mode <= 2 || mode >= 6) {
+    const int kind = mode % 6;
+    if (mode == 7 && (i & 3)) {
+      const int ua = (int)(r2 % 24), ub = (int)((r2 >> 8) % 12), uq = (int)((r2 >> 16) % 16);
+      const int eb = (i & 3) == 1 ? (ub < 6 ? ub : 2042 + ub - 6) : 1023 - 500 + (int)((r2 >> 24) % 1001);
+      const int ea = (i & 3) == 1   ? (ua < 4 ? ua : ua < 16 ? 100 + ua : 2040 + ua - 16)
+                                    : (uq < 8 ? 60 + uq : 1978 + uq - 8) + eb - 1023;  // the quotient's exponent
+      const uint64_t frac = 0x800FFFFFFFFFFFFFull;
+      a = bits_d((r0 & frac) | ((uint64_t)min(max(ea, 0), 2047) << 52));
+      b = bits_d((r1 & frac) | ((uint64_t)eb << 52));
+      if ((i & 3) == 3) {
+        a = bits_d(r0 & 0x8000000000000000ull);
+        b = bits_d((i & 4) ? r1 : r1 & frac);
+      }
+    } else if (kind == 0) {
       a = bits_d((r0 & 0x800FFFFFFFFFFFFFull) | ((uint64_t)(1023 - 60 + (int)(r2 % 121)) << 52));
       b = bits_d((r1 & 0x800FFFFFFFFFFFFFull) | ((uint64_t)(1023 - 60 + (int)((r2 >> 8) % 121)) << 52));
-    } else if (mode == 1) {
+    } else if (kind == 1) {
       a = bits_d(r0);
       b = bits_d(r1);
     } else {
@@ -1127,7 +1141,7 @@ __global__ void k_fp64_selftest(int mode, uint64_t seed, int64_t n, unsigned lon
       const double q = bits_d((r0 & 0x000FFFFFFFFFFFFFull) | ((uint64_t)(1023 - 30 + (int)((r2 >> 8) % 61)) << 52));
       a = bits_d(d_bits(__dmul_rn(b, q)) + (uint64_t)((int)((r2 >> 16) % 5) - 2));
     }
-    got = div_rn(a, b);
+    got = mode <= 2 ? div_rn(a, b) : div_by(a, b, __drcp_rn(b));
     want = __ddiv_rn(a, b);
   } else {
     if (mode == 3) {

@@ -111,6 +111,19 @@ __device__ __forceinline__ double div_rn(double a, double b) {
   return __longlong_as_double((long long)(sign | ((uint64_t)e << 52) | (m & kFp64Frac)));
 }
 
+// a / b from r = 1 / b (rounded to nearest): the product q = a r and one correction by q's remainder, which
+// the FMA forms exactly (P. Markstein, IBM J. Res. Dev. 34, 1990).  A chain of three FP64 operations where the
+// division takes ten, for a divisor used many times.  q is within two ulps, so the corrected quotient is a / b's
+// rounding but where a / b lies within 2^-50 ulps of the middle between two doubles.  a zero goes by the
+// product; where the quotient, its remainder or the reciprocal may leave the normal range, to the division.
+__device__ __forceinline__ double div_by(double a, double b, double r) {
+  const double q = a * r;
+  auto exponent = [](double x) { return (int)((uint64_t)__double_as_longlong(x) >> 52) & 0x7ff; };
+  const int ea = exponent(a), er = exponent(r), eq = exponent(q);
+  if (ea >= 110 && ea < 0x7ff && er > 0 && er < 0x7ff && eq >= 64 && eq <= 1982) return fma(fma(-q, b, a), r, q);
+  return a == 0.0 && er != 0x7ff ? q : a / b;
+}
+
 __device__ __forceinline__ double sqrt_rn(double x) {
   const uint64_t ux = (uint64_t)__double_as_longlong(x);
   const int ex = (int)(ux >> 52);  // the sign bit included: negative inputs land above 0x7ff

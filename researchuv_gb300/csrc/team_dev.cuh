@@ -9,17 +9,6 @@ namespace ruv {
 
 constexpr int kTeamDirect = 64;            // rows solved by the dense inverse (amg.cu kDirect)
 
-// a / b from r = 1 / b: the product and one correction by its exact remainder (the rounding of
-// the division up to the last bit; a chain of three FP64 operations, where the division takes ten).
-// Quotients that leave the normal range go to the division.
-__device__ __forceinline__ double div_by(double a, double b, double r) {
-  const double q = a * r;
-  if (a == 0.0) return q;
-  const int e = (int)((uint64_t)__double_as_longlong(q) >> 52) & 0x7ff;
-  if (e < 64 || e > 1982) return a / b;
-  return fma(fma(-q, b, a), r, q);
-}
-
 // sqrt(rr) <= norm, by its square (norm2 = square_of(norm)) where that is in range
 __device__ __forceinline__ double square_of(double norm) { return norm > 1e-140 && norm < 1e140 ? norm * norm : -1.0; }
 __device__ __forceinline__ bool at_most(double rr, double norm, double norm2) {
