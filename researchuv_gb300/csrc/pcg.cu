@@ -67,9 +67,9 @@ struct Tiles {
 // chart's tiles to arrive does it (every tile's sum is in global memory by then), combining the
 // partials in tile order as k_chart_step does -- the same bits whichever tile is last,
 // without a kernel of its own between the tile kernels (4 to 9 us each, five an iteration).
-enum : int { kStepNone = 0, kStepAlpha, kStepBeta, kStepBetaMixed, kStepAfterRefresh, kStepCheck64, kStepRz0, kStepBetaPc };
+enum : int { kStepAlpha, kStepBeta, kStepBetaMixed, kStepAfterRefresh, kStepCheck64, kStepRz0, kStepBetaPc };
 struct ChartStep {
-  int kind = kStepNone;
+  int kind = kStepAlpha;
   int precond_none = 0;  // rz is r.r
   int separate = 0;      // the preconditioner is applied by its own launches: beta comes after it
   int flexible = 0;
@@ -162,14 +162,24 @@ __device__ __forceinline__ void chart_step(const ChartStep& F, int64_t c, double
   }
 }
 
-// A tile's end: its sums v (thread 0's) into part, and the chart's step by the last tile.
+// A tile's end: its sums v (thread 0's) into part, and the chart's step by the last tile; or (NoStep, a kernel
+// of its own follows) the sums alone.
+struct NoStep {};
+template <int LPR, int U>
+constexpr bool steps_built() {
+  return (LPR <= 2 && U == 2) || (LPR == 8 && U == 4) || LPR >= 16;
+}
 template <int NV>
-__device__ __forceinline__ void tile_end(const Tiles& T, const ChartStep& F, int64_t t, int32_t ch, const double (&v)[NV],
+__device__ __forceinline__ void tile_end(const Tiles&, const NoStep&, int64_t t, int32_t, const double (&v)[NV],
                                          double* part) {
   if (threadIdx.x == 0)
 #pragma unroll
     for (int k = 0; k < NV; ++k) part[NV * t + k] = v[k];
-  if (F.kind == kStepNone) return;
+}
+template <int NV>
+__device__ __forceinline__ void tile_end(const Tiles& T, const ChartStep& F, int64_t t, int32_t ch, const double (&v)[NV],
+                                         double* part) {
+  tile_end<NV>(T, NoStep(), t, ch, v, part);
   const int64_t t0 = T.chart_tile[ch], n = T.chart_tile[ch + 1] - t0;
   if (n == 1) {
     if (threadIdx.x == 0) chart_step(F, ch, v[0], NV > 1 ? v[NV - 1] : 0.0);
@@ -339,14 +349,14 @@ __device__ __forceinline__ void spmv_pq_tile(int64_t beg, int64_t end, const int
 // per sub-warp in flight so a warp keeps U * K independent value/column loads and U * K
 // gathers outstanding.  Block-uniform trip counts keep every lane in the shuffles.  NW: the
 // column stream's kind (ColsWide, ColsNarrow, ColsRowRel).
-template <class S, int NR, int LPR, int U, int NW>
+template <class S, int NR, int LPR, int U, int NW, class Step>
 __global__ void __launch_bounds__(kTileThreads) k_spmv_pq_k(Tiles T, const ChartState* __restrict__ st,
                                                             const int32_t* __restrict__ row_ptr,
                                                             const int32_t* __restrict__ cols,
                                                             const uint16_t* __restrict__ c16,
                                                             const int32_t* __restrict__ cbase, const S* __restrict__ vals,
                                                             const S* __restrict__ p, S* __restrict__ q,
-                                                            double* __restrict__ part, ChartStep F) {
+                                                            double* __restrict__ part, Step F) {
   __shared__ S sh[32];
   const int64_t t = blockIdx.x;
   const int32_t ch = T.chart[t];
@@ -506,7 +516,7 @@ __global__ void __launch_bounds__(kTileThreads) k_spmv_tma(Tiles T, const ChartS
                                                            const uint16_t* __restrict__ c16,
                                                            const int32_t* __restrict__ cbase, const S* __restrict__ vals,
                                                            const S* __restrict__ p, S* __restrict__ q,
-                                                           double* __restrict__ part, ChartStep F) {
+                                                           double* __restrict__ part) {
   extern __shared__ __align__(16) unsigned char stage[];
   __shared__ S sh[32];
   const int64_t t = blockIdx.x;
@@ -533,28 +543,28 @@ __global__ void __launch_bounds__(kTileThreads) k_spmv_tma(Tiles T, const ChartS
   S accv[1] = {acc};
   block_sum_first<1, S>(accv, sh);
   const double v[1] = {(double)accv[0]};
-  tile_end<1>(T, F, t, ch, v, part);
+  tile_end<1>(T, NoStep(), t, ch, v, part);
 }
 
 // One launch of the SpMV for a column stream of kind nw (0 wide, 1 chart-relative, 2 row-
 // relative): the bulk-copy kernel when the context set it up (upload_tiles) and its stage fits,
 // else the CSR-vector kernel.
-template <class S, int NR, int LPR, int U, int NW>
+template <class S, int NR, int LPR, int U, int NW, class Step>
 void launch_spmv_nw(cudaStream_t s, unsigned grid, const Tiles& T, const ChartState* st, const int32_t* row_ptr,
                     const int32_t* cols, const uint16_t* c16, const int32_t* cbase, const S* vals, const S* p, S* q,
-                    double* part, const ChartStep& F) {
-  if constexpr (std::is_same<S, float>::value && NR == 2) {
+                    double* part, const Step& F) {
+  if constexpr (std::is_same<S, float>::value && NR == 2 && std::is_same<Step, NoStep>::value) {
     const size_t sm = spmv_tma_smem<S, NW>(T);
     if (T.max_rows > 0 && sm <= kSpmvTmaMaxSmem) {
-      k_spmv_tma<S, NR, LPR, U, NW><<<grid, kTileThreads, sm, s>>>(T, st, row_ptr, cols, c16, cbase, vals, p, q, part, F);
+      k_spmv_tma<S, NR, LPR, U, NW><<<grid, kTileThreads, sm, s>>>(T, st, row_ptr, cols, c16, cbase, vals, p, q, part);
       return;
     }
   }
   k_spmv_pq_k<S, NR, LPR, U, NW><<<grid, kTileThreads, 0, s>>>(T, st, row_ptr, cols, c16, cbase, vals, p, q, part, F);
 }
-template <class S, int NR, int LPR, int U>
+template <class S, int NR, int LPR, int U, class Step>
 void launch_spmv(cudaStream_t s, unsigned grid, const Tiles& T, const ChartState* st, const DevSystem& sys,
-                 const S* vals, const S* p, S* q, double* part, const ChartStep& F = ChartStep()) {
+                 const S* vals, const S* p, S* q, double* part, const Step& F) {
   if (sys.cols16 && sys.rowrel16)
     launch_spmv_nw<S, NR, LPR, U, 2>(s, grid, T, st, sys.row_ptr, sys.cols, sys.cols16, sys.cbase, vals, p, q, part, F);
   else if (sys.cols16)
@@ -579,12 +589,12 @@ void spmv_tma_attributes(const Tiles& T) {
 
 // x += alpha p; r -= alpha q; z = M^-1 r.  Partials: r.r, r.z.  precond: 0 = none (z = r),
 // 1 = Jacobi, 2 = applied separately afterwards (z is not written).
-template <class S, int NR>
+template <class S, int NR, class Step>
 __global__ void __launch_bounds__(kTileThreads) k_update(Tiles T, const ChartState* __restrict__ st,
                                                          const S* __restrict__ dinv, int use_jacobi,
                                                          S* __restrict__ x, S* __restrict__ r, S* __restrict__ z,
                                                          const S* __restrict__ p, const S* __restrict__ q,
-                                                         double* __restrict__ part, ChartStep F = ChartStep()) {
+                                                         double* __restrict__ part, Step F) {
   __shared__ S sh[2 * 32];
   int64_t t = blockIdx.x;
   const int32_t ch = T.chart[t];
@@ -683,7 +693,7 @@ __global__ void __launch_bounds__(kTileThreads) k_fold(Tiles T, const ChartState
 // r32 = r, z = M^-1 r (precond 0: z = r, 1: Jacobi, 2: applied separately, z not written).
 // Partials: r.r and r.z, summed in FP32 over r * rscale and rescaled per tile.  The CSR-vector
 // shape (LPR lanes, K = ceil(8 / LPR) slots, U rows in flight) is the tuned SpMV's.
-template <int NR, int LPR, int U, int NW>
+template <int NR, int LPR, int U, int NW, class Step>
 __global__ void __launch_bounds__(kTileThreads) k_true_residual(Tiles T, const ChartState* __restrict__ st,
                                                                 const int32_t* __restrict__ row_ptr,
                                                                 const int32_t* __restrict__ cols,
@@ -693,7 +703,7 @@ __global__ void __launch_bounds__(kTileThreads) k_true_residual(Tiles T, const C
                                                                 const float* __restrict__ bdf, const float* __restrict__ dinv,
                                                                 int precond, const float* __restrict__ xdf,
                                                                 float* __restrict__ r, float* __restrict__ z,
-                                                                double* __restrict__ part, ChartStep F) {
+                                                                double* __restrict__ part, Step F) {
   constexpr int K = (8 + LPR - 1) / LPR;
   __shared__ float sh[2 * 32];
   const int64_t t = blockIdx.x;
@@ -807,10 +817,10 @@ __global__ void __launch_bounds__(kTileThreads) k_true_residual(Tiles T, const C
 }
 
 // One launch of the true residual for the system's column stream kind.
-template <int NR, int LPR, int U, class MX>
+template <int NR, int LPR, int U, class MX, class Step>
 void launch_true_residual(cudaStream_t s, unsigned grid, const Tiles& T, const ChartState* st, const DevSystem& sys,
                           const MX& mx, const float* dinv32, int precond, float* r, float* z, double* part,
-                          const ChartStep& F) {
+                          const Step& F) {
 #define RUV_TR(NWV)                                                                                                   \
   k_true_residual<NR, LPR, U, NWV><<<grid, kTileThreads, 0, s>>>(T, st, sys.row_ptr, sys.cols, sys.cols16, sys.cbase, \
                                                                 sys.vals32, mx.vals_lo, mx.rsum, mx.bdf, dinv32,      \
@@ -821,10 +831,10 @@ void launch_true_residual(cudaStream_t s, unsigned grid, const Tiles& T, const C
 #undef RUV_TR
 }
 
-template <class S, int NR>
+template <class S, int NR, class Step>
 __global__ void __launch_bounds__(kTileThreads) k_dots_rz(Tiles T, const ChartState* __restrict__ st, const S* __restrict__ r,
                                                           const S* __restrict__ z, const S* __restrict__ q,
-                                                          double* __restrict__ part, ChartStep F = ChartStep()) {
+                                                          double* __restrict__ part, Step F) {
   __shared__ S sh[2 * 32];
   int64_t t = blockIdx.x;
   const int32_t ch = T.chart[t];
@@ -964,9 +974,17 @@ int32_t* arrived_counters(Ctx& ctx, int64_t n_charts) {
 }
 
 // Whether the tile kernels take the chart steps: up to eight tiles an SM.  With more, the fence and the
-// atomic that end every tile cost the kernels' throughput more than a kernel between them costs (4096
-// disks, 14,900 tiles: 110 against 106 ms; a 1024^2 field's 1,021 tiles 35.7 against 35.1).
-inline bool steps_in_tiles(const Ctx& ctx, int64_t n_tiles) { return n_tiles <= 8 * (int64_t)ctx.sm_count; }
+// atomic that end every tile cost the kernels' throughput as much as a kernel between them, or more (ms, in
+// the tiles / kernels between: one chart of 88,800 rows in FP64, 152 tiles, 10.5 / 10.9 for 400 iterations;
+// a 1024^2 field, 1,021 tiles, 28.6 / 28.8; 1,000 disks, 2,500 tiles, 14.8 / 15.0; a 1448^2 field, 2,048
+// tiles, 48.4 / 48.2; 4096 disks, 14,900 tiles, 99.8 / 99.6).  Only shapes that pick_shape takes, and not
+// the bulk-copy SpMV, are built with the steps; RUV_TILE_STEPS=1 / 0 takes them in the tiles whatever the
+// count / never (bit-identical results).
+template <int LPR, int U>
+bool steps_in_tiles(const Ctx& ctx, const Tiles& T) {
+  const char* e = std::getenv("RUV_TILE_STEPS");
+  return steps_built<LPR, U>() && T.max_rows == 0 && (e ? e[0] == '1' : T.n <= 8 * (int64_t)ctx.sm_count);
+}
 
 template <class S, int NR, int LPR, int U>
 void run_pcg(Ctx& ctx, DevSystem& sys, double* x64, const SolveOpts& o, Tiles T, ChartState* st, int* n_active,
@@ -1026,16 +1044,14 @@ void run_pcg(Ctx& ctx, DevSystem& sys, double* x64, const SolveOpts& o, Tiles T,
     base.st = st;
     base.n_active = n_active;
     base.arrived = arrived_counters(ctx, NC);
-    const bool in_tiles = steps_in_tiles(ctx, NTL);
-    auto step = [&](int kind) {
-      ChartStep f = base;
-      f.kind = in_tiles ? kind : kStepNone;
-      return f;
-    };
-    auto chart = [&](auto nv, int kind) {  // the step's own kernel where the tiles do not take it
-      if (in_tiles) return;
+    const bool in_tiles = steps_in_tiles<LPR, U>(ctx, T);
+    // a tile kernel and the chart step behind its sums: in the kernel, or in one of its own
+    auto with_step = [&](auto nv, int kind, auto launch) {
       ChartStep f = base;
       f.kind = kind;
+      if constexpr (steps_built<LPR, U>())
+        if (in_tiles) return launch(f);
+      launch(NoStep());
       k_chart_step<decltype(nv)::value><<<(unsigned)NC, kChartThreads, 0, s>>>(T, f, part);
     };
     constexpr std::integral_constant<int, 1> one{};
@@ -1045,16 +1061,19 @@ void run_pcg(Ctx& ctx, DevSystem& sys, double* x64, const SolveOpts& o, Tiles T,
     cudaGraphExec_t exec = nullptr;
     RUV_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     for (int rep = 0; rep < kCheckEvery; ++rep) {
-      launch_spmv<S, NR, LPR, U>(s, (unsigned)NTL, T, st, sys, vals, p, q, part, step(kStepAlpha));
-      chart(one, kStepAlpha);
-      k_update<S, NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, dinv, jac, mixed ? xs : reinterpret_cast<S*>(x64), r,
-                                                             z, p, q, part, step(mixed ? kStepBetaMixed : kStepBeta));
-      chart(two, mixed ? kStepBetaMixed : kStepBeta);
+      with_step(one, kStepAlpha, [&](const auto& f) {
+        launch_spmv<S, NR, LPR, U>(s, (unsigned)NTL, T, st, sys, vals, p, q, part, f);
+      });
+      with_step(two, mixed ? kStepBetaMixed : kStepBeta, [&](const auto& f) {
+        k_update<S, NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, dinv, jac, mixed ? xs : reinterpret_cast<S*>(x64), r,
+                                                               z, p, q, part, f);
+      });
       if (mixed) {
         k_fold<NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, 0, mx.xdf, reinterpret_cast<float*>(xs), x64);
-        launch_true_residual<NR, LPR, U>(s, (unsigned)NTL, T, st, sys, mx, dinv32, jac, reinterpret_cast<float*>(r),
-                                         reinterpret_cast<float*>(z), part, step(kStepAfterRefresh));
-        chart(two, kStepAfterRefresh);
+        with_step(two, kStepAfterRefresh, [&](const auto& f) {
+          launch_true_residual<NR, LPR, U>(s, (unsigned)NTL, T, st, sys, mx, dinv32, jac, reinterpret_cast<float*>(r),
+                                           reinterpret_cast<float*>(z), part, f);
+        });
       }
       k_direction<S, NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, z, p);
     }
@@ -1182,25 +1201,27 @@ void run_pcg_sep(Ctx& ctx, DevSystem& sys, double* x64, const SolveOpts& o, Tile
     base.n_active = n_active;
     base.done = done;
     base.arrived = arrived_counters(ctx, NC);
-    const bool in_tiles = steps_in_tiles(ctx, NTL);
-    auto step = [&](int kind) {
-      ChartStep f = base;
-      f.kind = in_tiles ? kind : kStepNone;
-      return f;
-    };
-    auto chart = [&](auto nv, int kind, const double* sums) -> int {  // (its own kernel, where the tiles do not)
-      if (in_tiles) return 0;
+    const bool in_tiles = steps_in_tiles<LPR, U>(ctx, T);
+    // a tile kernel and the chart step behind its sums: in the kernel, or in one of its own; the launches
+    auto with_step = [&](auto nv, int kind, const double* sums, auto launch) -> int {
       ChartStep f = base;
       f.kind = kind;
+      if constexpr (steps_built<LPR, U>())
+        if (in_tiles) {
+          launch(f);
+          return 1;
+        }
+      launch(NoStep());
       k_chart_step<decltype(nv)::value><<<(unsigned)NC, kChartThreads, 0, s>>>(T, f, sums);
-      return 1;
+      return 2;
+    };
+    auto dots = [&](const auto& f) {
+      k_dots_rz<S, NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, r, z, q, part2, f);
     };
     constexpr std::integral_constant<int, 1> one{};
     constexpr std::integral_constant<int, 2> two{};
-    k_dots_rz<S, NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, r, z, q, part2, step(kStepRz0));
-    count_launches(chart(two, kStepRz0, part2));
+    count_launches(1 + with_step(two, kStepRz0, part2, dots));
     k_copy_dir<S, NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, z, p);
-    count_launches(2);
     RUV_LAUNCH_CHECK();
     constexpr int kRep = 8;
     cudaGraph_t graph = nullptr;
@@ -1209,25 +1230,24 @@ void run_pcg_sep(Ctx& ctx, DevSystem& sys, double* x64, const SolveOpts& o, Tile
     RUV_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     for (int rep = 0; rep < kRep; ++rep) {
       int l = 0;
-      launch_spmv<S, NR, LPR, U>(s, (unsigned)NTL, T, st, sys, vals, p, q, part, step(kStepAlpha));
-      l += chart(one, kStepAlpha, part);
-      k_update<S, NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, dinv, 2, xiter, r, z, p, q, part,
-                                                             step(mixed ? kStepBetaMixed : kStepCheck64));
-      l += chart(two, mixed ? kStepBetaMixed : kStepCheck64, part);
+      l += with_step(one, kStepAlpha, part, [&](const auto& f) {
+        launch_spmv<S, NR, LPR, U>(s, (unsigned)NTL, T, st, sys, vals, p, q, part, f);
+      });
+      l += with_step(two, mixed ? kStepBetaMixed : kStepCheck64, part, [&](const auto& f) {
+        k_update<S, NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, dinv, 2, xiter, r, z, p, q, part, f);
+      });
       if (mixed) {
         k_fold<NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, 0, mx.xdf, reinterpret_cast<float*>(xs), x64);
-        launch_true_residual<NR, LPR, U>(s, (unsigned)NTL, T, st, sys, mx, dinv32, 2, reinterpret_cast<float*>(r),
-                                         reinterpret_cast<float*>(z), part, step(kStepAfterRefresh));
-        l += 2 + chart(two, kStepAfterRefresh, part);
+        l += 1 + with_step(two, kStepAfterRefresh, part, [&](const auto& f) {
+          launch_true_residual<NR, LPR, U>(s, (unsigned)NTL, T, st, sys, mx, dinv32, 2, reinterpret_cast<float*>(r),
+                                           reinterpret_cast<float*>(z), part, f);
+        });
       }
       to32();
-      l += 2 + conv;
-      l += P.apply(ctx, done);
+      l += conv + P.apply(ctx, done);
       to64();
-      k_dots_rz<S, NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, r, z, q, part2, step(kStepBetaPc));
-      l += chart(two, kStepBetaPc, part2);
+      l += 1 + with_step(two, kStepBetaPc, part2, dots);
       k_direction<S, NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, z, p);
-      l += 2;
       per_iter = l;
     }
     cudaError_t ce = cudaStreamEndCapture(s, &graph);
@@ -1393,12 +1413,12 @@ double time_spmv(Ctx& ctx, DevSystem& sys, Tiles T, int reps, int nbuf, bool ite
   const S* vals = std::is_same<S, float>::value ? reinterpret_cast<const S*>(sys.vals32) : reinterpret_cast<const S*>(sys.vals);
   auto launch = [&](int k) {
     launch_spmv<S, NR, LPR, U>(s, (unsigned)T.n, T, st, sys, vals, ps[k % nbuf],
-                               qs[k % nbuf], part);
+                               qs[k % nbuf], part, NoStep());
     count_launches(1);
     if (iter && T.n > 0) {
       k_update<S, NR><<<(unsigned)T.n, kTileThreads, 0, s>>>(T, st, nullptr, 2, xv, rv, nullptr, ps[k % nbuf],
-                                                             qs[k % nbuf], part2);
-      k_dots_rz<S, NR><<<(unsigned)T.n, kTileThreads, 0, s>>>(T, st, rv, rv, qs[k % nbuf], part2);
+                                                             qs[k % nbuf], part2, NoStep());
+      k_dots_rz<S, NR><<<(unsigned)T.n, kTileThreads, 0, s>>>(T, st, rv, rv, qs[k % nbuf], part2, NoStep());
       k_direction<S, NR><<<(unsigned)T.n, kTileThreads, 0, s>>>(T, st, rv, ps[k % nbuf]);
       count_launches(3);
     }
@@ -1760,7 +1780,7 @@ template <int LPR, int U>
 void na_iterations(cudaStream_t s, NoAllocScratch* S, Tiles T, const int32_t* row_ptr, const int32_t* cols,
                    const double* vals, double* x, int jac, int none, int64_t max_iter) {
   k_spmv_pq_k<double, 1, LPR, U, false><<<(unsigned)T.n, kTileThreads, 0, s>>>(T, &S->st, row_ptr, cols, nullptr, nullptr,
-                                                                              vals, S->p, S->q, S->part, ChartStep());
+                                                                              vals, S->p, S->q, S->part, NoStep());
   ChartStep f;
   f.precond_none = none;
   f.max_iter = max_iter;
@@ -1768,7 +1788,7 @@ void na_iterations(cudaStream_t s, NoAllocScratch* S, Tiles T, const int32_t* ro
   f.n_active = &S->n_active;
   f.kind = kStepAlpha;
   k_chart_step<1><<<1, kChartThreads, 0, s>>>(T, f, S->part);
-  k_update<double, 1><<<(unsigned)T.n, kTileThreads, 0, s>>>(T, &S->st, S->dinv, jac, x, S->r, S->z, S->p, S->q, S->part);
+  k_update<double, 1><<<(unsigned)T.n, kTileThreads, 0, s>>>(T, &S->st, S->dinv, jac, x, S->r, S->z, S->p, S->q, S->part, NoStep());
   f.kind = kStepBeta;
   k_chart_step<2><<<1, kChartThreads, 0, s>>>(T, f, S->part);
   k_direction<double, 1><<<(unsigned)T.n, kTileThreads, 0, s>>>(T, &S->st, S->z, S->p);
