@@ -2776,11 +2776,14 @@ class AmgPrecond final : public SepPrecond {
 };
 }  // namespace
 
-// The smoothers' weight on a chart's Laplacian (two right-hand sides).  Its edge weights are not negative, so
-// D^-1 A has no eigenvalue above 2 and any weight below 1 damps.  Iterations (max) and time at 0.6 / 0.667 /
-// 0.75 / 0.85 / 0.92 / 0.99: 4096 disks 32 / 30 / 28 / 26 / 26 / 40, 111 / 107 / 105 / 104 / 104 / 138 ms;
-// 1024^2 field 117 / 108 / 99 / 92 / 90 / 98, 37.6 / 35.1 / 33.0 / 31.1 / 31.2 / 33.2 ms.  A system from outside may
-// have larger eigenvalues and keeps 2/3, and so does a solve that asks for the first form's sums.
+// The smoothers' weight on a chart's Laplacian (two right-hand sides).  The assembled weights are not
+// negative, nor are those of a level below a tentative prolongator, so D^-1 A has no eigenvalue above 2
+// there and any weight below 1 damps.  Below a smoothed prolongator nothing bounds them, but 0.85 damps up to 2.35:
+// the largest measured on any level was 1.997, on stretched, jittered, graded and Delaunay charts of 8,000
+// to 40,000 rows.  Iterations (max) and time at 0.6 / 0.667 / 0.75 / 0.85 / 0.92 / 0.99: 4096 disks
+// 32 / 30 / 28 / 26 / 26 / 40, 111 / 107 / 105 / 104 / 104 / 138 ms; 1024^2 field 117 / 108 / 99 / 92 / 90 / 98,
+// 37.6 / 35.1 / 33.0 / 31.1 / 31.2 / 33.2 ms.  A system from outside may have larger eigenvalues and keeps 2/3,
+// and so does a solve that asks for the first form's sums.
 constexpr float kOmegaChart = 0.85f;
 std::unique_ptr<SepPrecond> make_amg(Ctx& ctx, const DevSystem& sys, bool smooth, bool first_form) {
   return std::unique_ptr<SepPrecond>(

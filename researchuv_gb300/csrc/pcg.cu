@@ -1382,7 +1382,9 @@ Shape pick_shape(const Ctx& ctx, const DevSystem& sys, bool one_lane = false) {
   int lpr = ctx.lanes_per_row > 0 ? ctx.lanes_per_row : (avg <= 8 ? 2 : avg <= 12 ? 8 : avg <= 24 ? 16 : 32);
   int u = ctx.unroll > 0 ? ctx.unroll : (lpr <= 4 ? 2 : lpr == 8 ? 4 : 1);
   // FP64: one lane per row, whose sum needs no additions across lanes (a quarter of a two-lane row's FP64
-  // instructions): 49.0 -> 47.5 ms on an 89,401-row chart, 14.9 -> 14.3 ms on 160,000 rows
+  // instructions).  Solves, two lanes / one (ms): Jacobi, one chart of 89,401 rows 41.5 / 38.2, of 357,604
+  // 152 / 138; AMG-SA, of 1.0 million 24.7 / 24.2, 2.1 million 38.5 / 37.5, 4.2 million 71.9 / 69.8, 4096 disks of
+  // 14.4 million 90.8 / 87.2
   if (one_lane && ctx.lanes_per_row == 0 && lpr == 2) lpr = 1;
   return Shape{lpr, u};
 }

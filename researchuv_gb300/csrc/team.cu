@@ -517,8 +517,10 @@ struct TeamSys {
   int store_bytes;  // dynamic shared memory for a CTA's rows of the operator
 };
 
-// CTAs on an SM: the FP32 loop without a preconditioner of its own fits 64 registers a thread; the others
-// take 128 (spilled values would come back from L2, past an L1 that every cluster barrier empties).
+// CTAs on an SM: the FP32 loop without a preconditioner of its own runs at 64 registers a thread, the others
+// at 128.  Three of them spill (bytes a thread, stores / loads: k_team<float,2,0> 92 / 172, <float,2,1> 120 / 156,
+// <double,2,2> 160 / 160; the rest 48 and less), and what is spilled comes back from L2, past an L1 that every
+// cluster barrier empties.
 template <class S, int PCK>
 constexpr int team_per_sm() {
   return std::is_same<S, float>::value && PCK == 0 ? 2 : 1;
