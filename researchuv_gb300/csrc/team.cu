@@ -980,14 +980,24 @@ int64_t team_solve(Ctx& ctx, const DevSystem& sys, TeamLoop<S> loop, const TeamP
   loop.spin_limit = le ? std::max<int64_t>(0, std::atoll(le)) : kTeamSpin;
   const char* re = std::getenv("RUV_TEAM_ROWS");
   // The largest chart a team of 16 SMs takes, where both ways were measured (ms, team / launch loop):
-  // mixed Jacobi 39,000 rows 21.8 / 31.9, 89,000 57 / 60, 128,000 121 / 102; FP64 Jacobi, two columns,
-  // 19,000 rows 16.2 / 19.4, 39,000 37 / 27, one column half the arithmetic; V-cycle 32,000 rows mixed
-  // 5.8 / 6.4, FP64 6.2 / 6.6, 89,000 mixed 11.9 / 9.4; colour-ordered IC(0) 14,400 rows 7.0 / 35.
-  const int64_t most = re                ? std::atoll(re)
-                       : kind == 1       ? (mixed ? 40000 : 32000)
-                       : kind == 2       ? (mixed ? 90000 : 40000)
-                       : mixed           ? 90000
-                                         : 48000 / NR;
+  // mixed Jacobi 47,500 rows 20.5 / 27.3, 66,600 31.1 / 33.3, 88,800 44.7 / 42.3; FP64 Jacobi, two columns,
+  // 16,400 rows 11.3 / 14.8, 21,900 15.5 / 17.0, 25,000 20.4 / 18.0; V-cycle 32,000 rows mixed 5.8 / 6.4, FP64
+  // 6.2 / 6.6, 89,000 mixed 11.9 / 9.4; colour-ordered IC(0) 14,400 rows 7.0 / 35.
+  // One column: rows of at most 8 entries cost the loop one lane each, and the line lies at about as many
+  // entries (7.5 a row, 25,000 rows 15.7 / 15.8, 30,000 16.6 / 16.2, 40,000 20.1 / 16.5; 5 a row, 40,000 rows
+  // 13.9 / 14.0, 47,000 20.5 / 18.8), longer rows eight lanes and more (10 a row, 40,000 rows 21.3 / 23.4, 47,000
+  // 24.1 / 23.2).  A team gives a row one thread whatever its length, so long rows lower every limit: Jacobi 47
+  // entries a row, 40,000 rows 28.4 / 30.9; 94, 20,000 rows 11.0 / 11.8, 25,000 15.8 / 14.1, 40,000 29.8 / 21.1;
+  // 187, 10,000 rows 6.0 / 6.5, 15,000 9.3 / 9.0.  V-cycle 47, 10,000 rows 6.6 / 7.2; 94, 5,000 rows 10.9 / 11.4,
+  // 10,000 15.7 / 14.1, 30,000 24.0 / 16.8.  IC(0) 24, 40,000 rows 240 / 249; 47, 40,000 rows 475 / 459.
+  const double per_row = sys.n_rows > 0 ? std::max(1.0, (double)sys.nnz / (double)sys.n_rows) : 1.0;
+  const int64_t by_rows = kind == 1   ? (mixed ? 40000 : 32000)
+                          : kind == 2 ? (mixed ? 90000 : 40000)
+                          : mixed     ? 75000
+                          : NR == 2   ? 23000
+                                      : 43000;
+  const double entries = kind == 1 ? 5e5 : kind == 2 ? 1.5e6 : !mixed && NR == 1 && per_row <= 8.0 ? 2e5 : 2e6;
+  const int64_t most = re ? std::atoll(re) : std::min(by_rows, (int64_t)(entries / per_row));
   // a V-cycle is a chain of small steps, and a chart left to the other loop makes them all again: all
   // charts by teams, or none.  Teams hold 512 rows in flight on an SM where the launch loop's kernels
   // stream: 473,000 rows in 300 charts took 146 us an iteration against 172, 14.4 million 7,000 against
@@ -1063,7 +1073,6 @@ int64_t team_solve(Ctx& ctx, const DevSystem& sys, TeamLoop<S> loop, const TeamP
     cudaStream_t s = --classes == 0 ? main : ctx.team_stream[join.used++];
     const TeamSys A{d_order + first[k], sys.chart_row, sys.row_ptr, sys.cols, sys.cols16, sys.cbase, nw, 0};
     const int64_t rows = rows_of(order[first[k]]);  // the class's largest
-    const double per_row = (double)sys.nnz / (double)sys.n_rows;
     if (kind == 1) launch_team<S, NR, 1>(s, 1 << k, n, rows, per_row, A, loop, pc);
     else if (kind == 2) launch_team<S, NR, 2>(s, 1 << k, n, rows, per_row, A, loop, pc);
     else launch_team<S, NR, 0>(s, 1 << k, n, rows, per_row, A, loop, pc);
