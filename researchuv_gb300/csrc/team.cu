@@ -911,7 +911,6 @@ __global__ void __launch_bounds__(kTeamThreads, team_per_sm<S, PCK>())
 }
 
 // ---------------------------------------------------------------- which charts, and how many CTAs
-constexpr int64_t kTeamAmgRows = 600000;
 // CTAs of a team for `want` CTAs' worth of work.
 int team_ctas(int64_t want) {
   int c = 1;
@@ -1000,10 +999,23 @@ int64_t team_solve(Ctx& ctx, const DevSystem& sys, TeamLoop<S> loop, const TeamP
   const int64_t most = re ? std::atoll(re) : std::min(by_rows, (int64_t)(entries / per_row));
   // a V-cycle is a chain of small steps, and a chart left to the other loop makes them all again: all
   // charts by teams, or none.  Teams hold 512 rows in flight on an SM where the launch loop's kernels
-  // stream: 473,000 rows in 300 charts took 146 us an iteration against 172, 14.4 million 7,000 against
-  // 2,900.
-  const bool none = !teams_on(ctx) || (pc && kind == 0) ||
-                    (kind == 1 && (largest > most || sys.n_rows > kTeamAmgRows));
+  // stream, so a batch of many rows is the other loop's, and the sooner the larger its charts are, whose
+  // teams of 16 SMs then wait for each other (ms, team / loop, at a largest chart and rows in all).  AMG-SA mixed: 8,000
+  // 646,000 8.1 / 8.5; 10,000 517,000 6.9 / 7.2, 609,000 8.2 / 7.9; 14,500 375,000 6.7 / 7.0, 555,000 8.9 / 8.3; 18,500
+  // 335,000 6.3 / 6.9, 446,000 8.0 / 7.5; 24,000 404,000 7.8 / 7.7, 518,000 9.0 / 8.0.  AMG-SA FP64: 4,000 635,000 8.9 / 9.5;
+  // 5,900 466,000 7.3 / 7.6; 8,000 212,000 4.7 / 5.5, 440,000 7.7 / 7.4; 10,000 167,000 4.9 / 5.1, 320,000 7.2 / 6.5; 23,500
+  // 231,000 6.3 / 6.8, 348,000 8.3 / 7.8.  Tentative prolongators, cheaper cycles and more of them: mixed 14,900 691,000
+  // 10.4 / 11.4, 19,400 446,000 8.5 / 9.1, 588,000 11.5 / 10.4; FP64 10,000 254,000 6.7 / 8.4, 517,000 11.4 / 11.5, 23,500 333,000
+  // 9.1 / 10.2, 583,000 15.1 / 13.2.
+  bool none = !teams_on(ctx) || (pc && kind == 0);
+  if (kind == 1) {
+    const bool sa = pc->amg.lv[0].smoothed != 0;
+    const int64_t line = sa ? (mixed ? 10000 : 6000) : (mixed ? 16000 : 10000);
+    const int64_t rows = largest <= line ? (sa || mixed ? 600000 : 500000)
+                         : sa            ? (mixed ? 400000 : 250000)
+                                         : (mixed ? 450000 : 350000);
+    none = none || largest > most || sys.n_rows > rows;
+  }
   // Rows per CTA: as few as let every team run at once.  An FP32 step of one CTA of 512 threads costs
   // little more for two rows a thread, and its block barrier tens of clocks where a cluster's takes
   // over a thousand; FP64 rows are bound by the SM's FP64 pipe and spread out earlier.
