@@ -46,10 +46,12 @@ constexpr float kOmega = 2.0f / 3.0f;
 constexpr int kPairRounds = 3;
 // From this many rows on, a level's matching passes take two rounds and a third level gets a smoothed
 // prolongator: set-up and cycles stream HBM there, and what they save is more than the iterations they
-// cost (4096 disks: set-up 29.3 -> 24.6 ms, iterations 26 / 15.4 -> 27 / 17.9, solve 103.2 -> 99.1 ms; 1024^2
-// field 92 -> 87 iterations, 30.7 -> 28.4 ms).  Below, steps cost their latency whatever their rows, and
-// iterations count: a 300^2 chart 52 -> 62 iterations, 11.9 -> 13.0 ms.
-constexpr int64_t kLargeRows = 500000;
+// cost (ms, three rounds and two levels / two and three, launch loop.  4096 disks, 14.4 million rows: 104.6 / 102.2,
+// set-up 27.8 / 24.0, iterations 26 / 15.2 and 28 / 17.6; 1,000 disks, 3.6 million, 28.8 / 28.0; a 1448^2 field, 2.1 million, 36.4 /
+// 35.4).  With fewer rows or smaller charts iterations count: disks of up to 20,000 triangles, 2.25 million
+// rows 18.4 / 19.1, 1.1 million 11.2 / 11.5; of up to 50,000, 2.2 million 19.5 / 19.6, 0.9 million 11.05 / 11.27; 1024^2 fields
+// 20.7 / 21.8 and 19.95 / 19.98; a 300^2 chart 11.9 / 13.0.
+constexpr int64_t kLargeRows = 3000000;
 constexpr int kLargeRounds = 2, kLargeSaLevels = 3;
 // distinct keys per accumulated strength row: group strengths beyond it (only on dense coarse
 // levels of the smoothed hierarchy) are left out of the matching, deterministically
