@@ -1023,7 +1023,7 @@ void run_pcg(Ctx& ctx, DevSystem& sys, double* x64, const SolveOpts& o, Tiles T,
   // the charts a team solves in one kernel (team.cu); the loop below takes the others
   int64_t left = NTL > 0 ? 1 : 0;
   if constexpr (std::is_same<S, double>::value || NR == 2) {
-    if (left && o.teams) {
+    if (left && o.teams && o.max_iter > -kCheckEvery) {  // (the loop below replays nothing under that)
       const TeamLoop<S> loop{vals, dinv, mixed ? xs : reinterpret_cast<S*>(x64), r, z, p, q, x64, nullptr, nullptr, mx.vals_lo, mx.rsum, mx.bdf, mx.xdf, st, n_active,
                              o.max_iter, refresh_delta(), jac};
       left = team_solve<S, NR>(ctx, sys, loop, nullptr);
@@ -1168,10 +1168,11 @@ void run_pcg_sep(Ctx& ctx, DevSystem& sys, double* x64, const SolveOpts& o, Tile
   k_chart_init<<<(unsigned)NC, kChartThreads, 0, s>>>(T, st, part, o.tol, 0, n_active);  // (rz replaced below)
   count_launches(1);
   RUV_LAUNCH_CHECK();
+  constexpr int kRep = 8;  // iterations of a graph
   // the charts a team solves in one kernel (team.cu); the loop below takes the others
   int64_t left = NTL > 0 ? 1 : 0;
   if constexpr (std::is_same<S, double>::value || NR == 2) {
-    if (left && o.teams) {
+    if (left && o.teams && o.max_iter > -kRep) {  // (the loop below replays nothing under that)
       const TeamLoop<S> loop{vals, dinv, xiter, r, z, p, q, x64, r32, z32, mx.vals_lo, mx.rsum, mx.bdf, mx.xdf, st, n_active,
                              o.max_iter, refresh_delta(), 0};
       TeamPrecond tp;
@@ -1223,7 +1224,6 @@ void run_pcg_sep(Ctx& ctx, DevSystem& sys, double* x64, const SolveOpts& o, Tile
     count_launches(1 + with_step(two, kStepRz0, part2, dots));
     k_copy_dir<S, NR><<<(unsigned)NTL, kTileThreads, 0, s>>>(T, st, z, p);
     RUV_LAUNCH_CHECK();
-    constexpr int kRep = 8;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     int per_iter = 0;
