@@ -888,6 +888,9 @@ __global__ void __launch_bounds__(kChartThreads) k_chart_init(Tiles T, ChartStat
   } else if (sqrt(v[0]) <= s.tol_abs) {
     s.status = RUV_OK;
     s.state = kDone;
+  } else if (T.chart_tile[c] == T.chart_tile[c + 1]) {
+    s.status = RUV_ERR_BREAKDOWN;  // no rows under a tolerance that zero does not meet: p.q is 0, and no tile takes that step
+    s.state = kDone;
   } else {
     s.status = RUV_ERR_NOT_CONVERGED;
     s.state = kActive;

@@ -544,7 +544,7 @@ __global__ void __launch_bounds__(kTeamThreads, team_per_sm<S, PCK>())
   tm.bars = 0;
   const int chart = A.order[cluster_id()];
   auto set_due = [&](double norm) {
-    sh.due = fmax(norm, sh.st.tol_abs);
+    sh.due = mixed ? fmax(norm, sh.st.tol_abs) : sh.st.tol_abs;  // (FP64: a tolerance below zero is met by nothing)
     sh.due2 = square_of(sh.due);
   };
   if (threadIdx.x < kTeamMaxCtas) sh.left[threadIdx.x] = kStaying;
