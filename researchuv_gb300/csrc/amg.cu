@@ -44,14 +44,21 @@ constexpr float kOmega = 2.0f / 3.0f;
 // save about 2.3 ms of set-up on the 4096-disk step and 11 ms on the 2048^2 field's step
 // (fewer iterations there too: 130 against 138)
 constexpr int kPairRounds = 3;
-// From this many rows on, a level's matching passes take two rounds and a third level gets a smoothed
-// prolongator: set-up and cycles stream HBM there, and what they save is more than the iterations they
+// From this many rows on, or with a chart of that many, a level's matching passes take two rounds and a third level gets a
+// smoothed prolongator: set-up and cycles stream HBM there, and what they save is more than the iterations they
 // cost (ms, three rounds and two levels / two and three, launch loop.  4096 disks, 14.4 million rows: 104.6 / 102.2,
-// set-up 27.8 / 24.0, iterations 26 / 15.2 and 28 / 17.6; 1,000 disks, 3.6 million, 28.8 / 28.0; a 1448^2 field, 2.1 million, 36.4 /
-// 35.4).  With fewer rows or smaller charts iterations count: disks of up to 20,000 triangles, 2.25 million
-// rows 18.4 / 19.1, 1.1 million 11.2 / 11.5; of up to 50,000, 2.2 million 19.5 / 19.6, 0.9 million 11.05 / 11.27; 1024^2 fields
-// 20.7 / 21.8 and 19.95 / 19.98; a 300^2 chart 11.9 / 13.0.
-constexpr int64_t kLargeRows = 3000000;
+// set-up 27.8 / 24.0, iterations 26 / 15.2 and 28 / 17.6; 1,000 disks, 3.6 million, 28.8 / 28.0; one chart, means over
+// height fields: 2.1 million rows 36.4 / 35.2, 1.56 million 28.0 / 27.4, 1.32 million 32.0 / 30.7).  With fewer rows or smaller charts
+// iterations count: one chart, 1.05 million rows 24.9 / 25.3 (twelve fields, each way by up to a tenth), 0.8 million 21.1 / 21.3,
+// 0.5 million 13.6 / 14.8; fields of up to 1,050,000 rows, 1.0 to 1.6 million in all, 26.4 / 27.0; disks of up to 20,000
+// triangles, 2.25 million rows 18.4 / 19.1, 1.1 million 11.2 / 11.5; of up to 50,000, 2.2 million 19.5 / 19.6, 0.9 million 11.05 / 11.27.
+constexpr int64_t kLargeRows = 3000000, kLargeChart = 1200000;
+bool large_level(int64_t rows, const std::vector<int64_t>& chart_row) {
+  if (rows >= kLargeRows) return true;
+  int64_t most = 0;
+  for (size_t c = 0; c + 1 < chart_row.size(); ++c) most = std::max(most, chart_row[c + 1] - chart_row[c]);
+  return most >= kLargeChart;
+}
 constexpr int kLargeRounds = 2, kLargeSaLevels = 3;
 // distinct keys per accumulated strength row: group strengths beyond it (only on dense coarse
 // levels of the smoothed hierarchy) are left out of the matching, deterministically
@@ -2022,7 +2029,7 @@ AmgHierarchy* amg_setup(Ctx& ctx, const DevSystem& sys, bool smooth, std::string
   // smoothed prolongators on the first sa_levels levels, tentative below (the coarse levels of a
   // smoothed hierarchy are the densest: their products and cycles cost the most)
   const bool by_size = !first_form;
-  H->sa_levels = !smooth ? 0 : by_size && sys.n_rows >= kLargeRows ? kLargeSaLevels : kSaLevels;
+  H->sa_levels = !smooth ? 0 : by_size && large_level(sys.n_rows, sys.h_chart_row) ? kLargeSaLevels : kSaLevels;
   if (const char* e = std::getenv("RUV_AMG_SA_LEVELS")) H->sa_levels = smooth ? std::max(0, std::atoi(e)) : 0;
   H->alpha_c = 1.5f;  // over-correct the piecewise-constant coarse space of tentative levels
   if (const char* e = std::getenv("RUV_AMG_ALPHA")) H->alpha_c = (float)std::atof(e);
@@ -2109,7 +2116,7 @@ AmgHierarchy* amg_setup(Ctx& ctx, const DevSystem& sys, bool smooth, std::string
     if (n_cont == 0) break;
     // ---- aggregation: pairs of rows, then pairs of pairs
     const int rounds = rounds_env ? std::max(1, std::atoi(rounds_env))
-                       : by_size && L.n >= kLargeRows ? kLargeRounds : kPairRounds;
+                       : by_size && large_level(L.n, L.h_chart_row) ? kLargeRounds : kPairRounds;
     int32_t* mate = ctx.ws.get<int32_t>(tag + ".mate", L.n);
     int32_t* prop = ctx.ws.get<int32_t>(tag + ".prop", L.n);
     RUV_CUDA(cudaMemsetAsync(mate, 0xff, sizeof(int32_t) * L.n, s));

@@ -95,3 +95,25 @@ def test_the_weight_damps_on_every_level(monkeypatch, sx, jitter, graded, smooth
                 x = y
             assert np.linalg.norm(x) < 2.0 / 0.85, (sa, k)
             k += 1
+
+
+@pytest.mark.parametrize("ns,large", [((1098,), True), ((1097,), False), ((1000, 600, 600), False)])
+def test_large_form_by_the_largest_chart(monkeypatch, ns, large):
+    vo, to, p3, tr = [0], [0], [], []
+    for k, n in enumerate(ns):
+        p, f = W.height_field(n, 8, 0.15, seed=5 + k)
+        p3.append(p)
+        tr.append(f)
+        vo.append(vo[-1] + len(p))
+        to.append(to[-1] + len(f))
+    C = R.prepare_patches(np.array(vo), np.array(to), np.concatenate(p3), np.concatenate(tr))
+    out = []
+    for form in ({}, SMALL):
+        for knob, v in form.items():
+            monkeypatch.setenv(knob, v)
+        out.append(R.unfold_charts(R.Context(0), C, R.UnfoldOptions(precond=R.Precond.AMG_SA)))
+    assert (out[0][0].n_free >= 1200000) == large
+    for a, b in zip(*out):
+        assert a.status == R.Status.OK and b.status == R.Status.OK
+        assert np.array_equal(a.uv, b.uv) != large
+        assert O.uv_error(a.uv, b.uv) <= 1e-6
