@@ -21,7 +21,9 @@
 #include "team_dev.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
+#include <functional>
 
 namespace ruv {
 namespace {
@@ -1015,6 +1017,32 @@ int64_t team_solve(Ctx& ctx, const DevSystem& sys, TeamLoop<S> loop, const TeamP
                          : sa            ? (mixed ? 400000 : 250000)
                                          : (mixed ? 450000 : 350000);
     none = none || largest > most || sys.n_rows > rows;
+  }
+  // IC(0): a team of one CTA an SM has its chart's levels for itself, where the loop's sweeps hold several charts
+  // an SM and end with the longest.  So batches whose charts wait for each other's SMs are the loop's: by
+  // `waves`, the time of all teams over the longest chart's, a chart's taken as rows^1.25 (team / loop ms at waves.  Natural
+  // order mixed: 1 5.9 / 8.9, 1.3 9.4 / 12.1, 1.5 4.2 / 4.5, 1.95 13.1 / 12.5, 2.6 56.8 / 40.7, 20,000 charts 108 / 44; FP64: 1 15.6 / 18.4,
+  // 1.3 19.1 / 18.9, 1.5 7.5 / 6.8, 1.95 27.4 / 19.6, 20,000 charts 216 / 79.  Colours, whose levels are wide and few, teams of
+  // one CTA mixed: 6 4.6 / 5.5, 26 16.7 / 16.8, 39 9.2 / 9.0; FP64: 5 22.0 / 25.1, 6 6.7 / 6.5, 26 25.6 / 21.9; of two mixed: 1.5 32.7 / 39.2, 1.8
+  // 49.8 / 48.0; FP64: 1.5 44.9 / 51.6, 1.7 55.7 / 53.5; of four mixed: 1.2 44.8 / 41.2, 1.5 64.9 / 73.8, 1.75 83 / 80; FP64: 1 67 / 82,
+  // 1.2 59.7 / 53.6, 1.5 93 / 91; of eight: 1.5 120 / 171 mixed, 161 / 208 FP64, 2.9 194 / 192 and 273 / 226; of sixteen
+  // 2.2 122 / 270, 162 / 332).
+  if (kind == 2 && !re && !none) {
+    const bool colours = pc->ic0.to_orig != nullptr;
+    const int ctas = team_ctas(std::max<int64_t>(1, pc->ic0.width / 256));
+    const size_t slots = (size_t)std::max(1, ctx.sm_count / ctas);
+    std::vector<double> cost;
+    for (int64_t c = 0; c < NC; ++c)
+      if (rows_of(c) > 0 && rows_of(c) <= most) cost.push_back(std::pow((double)rows_of(c), 1.25));
+    std::sort(cost.begin(), cost.end(), std::greater<double>());
+    double waves = 1.0, sum = 0.0;
+    for (double c : cost) sum += c;
+    if (cost.size() > slots) waves = std::max(sum / (double)slots, cost[slots - 1] + cost[slots]) / cost[0];
+    none = waves > (!colours    ? (mixed ? 1.6 : 1.25)
+                    : ctas == 1 ? (mixed ? 20.0 : 5.5)
+                    : ctas == 2 ? (mixed ? 1.7 : 1.55)
+                    : ctas == 4 ? (mixed ? 1.5 : 1.1)
+                                : (mixed ? 2.8 : 2.1));
   }
   // Rows per CTA: as few as let every team run at once.  An FP32 step of one CTA of 512 threads costs
   // little more for two rows a thread, and its block barrier tens of clocks where a cluster's takes
