@@ -342,6 +342,40 @@ __global__ void __launch_bounds__(kMetThreads) k_chart_metrics(const int64_t* __
   out[5 * c + 4] = (double)(sums[2] < 0.0 ? counts[3] : counts[2]);
 }
 
+// The same sums with a thread per chart, for batches of many short charts: there the FP64 pipe bounds the
+// kernel above, whose additions are one lane of a warp instruction each (20 clocks of an SM), and 32
+// charts share an instruction here, but the longest chart's walk through global memory bounds it.  The line by
+// triangles in all over the longest chart's (ms a call, this / above): 300 charts of 197 longest ones 0.099 / 0.083, 1,000 of 470
+// 0.251 / 0.193, 3,000 of 1,200 2.19 / 1.85, 3,000 of 1,428 0.410 / 0.425, 3,000 of 2,023 0.153 / 0.189, 30,000 of
+// 20,423 0.79 / 1.29.
+constexpr int64_t kMetEach = 1400;
+__global__ void k_chart_metrics_each(int64_t n_charts, const int64_t* __restrict__ tri_off,
+                                     const double4* __restrict__ m, double* __restrict__ out) {
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= n_charts) return;
+  double cs = 0.0, cm = 0.0, as = 0.0, sg = 0.0;
+  int64_t cnt = 0, flips = 0, le = 0, ge = 0;
+  for (int64_t t = tri_off[c]; t < tri_off[c + 1]; ++t) {
+    const double4 r = m[t];
+    if (r.x >= 0.0) {
+      cs = ad(cs, r.x);
+      cm = rmax(cm, r.x);
+      as = ad(as, r.y);
+      ++cnt;
+    }
+    flips += r.z != 0.0;
+    le += r.w <= 0.0;
+    ge += r.w >= 0.0;
+    sg = ad(sg, r.w);
+  }
+  const double nd = (double)(cnt > 1 ? cnt : 1);
+  out[5 * c] = dv(cs, nd);
+  out[5 * c + 1] = cm;
+  out[5 * c + 2] = dv(as, nd);
+  out[5 * c + 3] = (double)flips;
+  out[5 * c + 4] = (double)(sg < 0.0 ? ge : le);
+}
+
 // ---------------------------------------------------------------- rectangularize (metrics.rs:147-227)
 constexpr int kRectAngles = 72;
 constexpr int kRectThreads = 512;
@@ -663,7 +697,12 @@ void chart_metrics(Ctx& ctx, const DevBatch& bt, const double* uv, std::vector<d
     count_launches(1);
   }
   if (NC > 0) {
-    k_chart_metrics<<<(unsigned)NC, kMetThreads, 0, s>>>(bt.tri_off, m, o);
+    int64_t longest = 0;
+    for (int64_t c = 0; c < NC; ++c) longest = std::max(longest, bt.h_tri_off[c + 1] - bt.h_tri_off[c]);
+    if (NT > kMetEach * longest)
+      k_chart_metrics_each<<<div_up(NC, 64), 64, 0, s>>>(NC, bt.tri_off, m, o);
+    else
+      k_chart_metrics<<<(unsigned)NC, kMetThreads, 0, s>>>(bt.tri_off, m, o);
     count_launches(1);
   }
   RUV_LAUNCH_CHECK();
